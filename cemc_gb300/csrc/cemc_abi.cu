@@ -20,6 +20,7 @@
 
 #include "cemc_field.h"
 #include "cemc_kernels.h"
+#include "cemc_sched.h"
 #include "cemc_spin.h"
 
 namespace {
@@ -292,6 +293,12 @@ extern "C" int cemc_geometry_create(const cemc_geometry_desc *d, cemc_geometry *
   std::vector<int32_t> table_pad((size_t)N * cpad);
   for (int i = 0; i < N; ++i)
     for (int c = 0; c < cpad; ++c) table_pad[(size_t)i * cpad + c] = d->table[(size_t)i * C + (c < C ? c : 0)];
+  // the rows in 16 bits for the scheduled kernel (spin basis only: its rows are one cp.async ring entry)
+  const int cp16 = (C + 7) & ~7;
+  const bool has16 = N <= 65536 && B == 1 && G == 1 && C <= CEMC_SPIN_MAX_COLS;
+  std::vector<uint16_t> table16(has16 ? (size_t)N * cp16 : 1);
+  for (int i = 0; has16 && i < N; ++i)
+    for (int c = 0; c < cp16; ++c) table16[(size_t)i * cp16 + c] = (uint16_t)d->table[(size_t)i * C + (c < C ? c : 0)];
   std::vector<int32_t> table_cm((size_t)N * C);
   for (int i = 0; i < N; ++i)
     for (int c = 0; c < C; ++c) table_cm[(size_t)c * N + i] = d->table[(size_t)i * C + c];
@@ -642,6 +649,7 @@ extern "C" int cemc_geometry_create(const cemc_geometry_desc *d, cemc_geometry *
       {qtr_shift.data(), qtr_shift.size(), 0},
       {qtr_lane_term.data(), 9 * 4, 0},
       {qtr_lane_first.data(), 8 * 4, 0},
+      {table16.data(), table16.size() * 2, 0},
   };
   size_t total = 0;
   for (auto &p : parts) {
@@ -676,6 +684,8 @@ extern "C" int cemc_geometry_create(const cemc_geometry_desc *d, cemc_geometry *
   g.n_slots = n_slots;
   g.cpad = cpad;
   g.table = reinterpret_cast<const int32_t *>(base + parts[0].off);
+  g.table16 = has16 ? reinterpret_cast<const uint16_t *>(base + parts[39].off) : nullptr;
+  g.cp16 = cp16;
   g.table_cm = reinterpret_cast<const int32_t *>(base + parts[1].off);
   g.terms = reinterpret_cast<const uint16_t *>(base + parts[2].off);
   g.lane_term = reinterpret_cast<const int32_t *>(base + parts[3].off);
@@ -768,6 +778,61 @@ extern "C" size_t cemc_stamp_words(const cemc_geometry *geo, int32_t n_chains) {
   while ((1 << bits) < geo->g.n_sites) ++bits;
   return 2 * ((size_t)1 << bits) * (size_t)n_chains;
 }
+
+namespace {
+
+// Shape of the scheduled kernel for this geometry, or false where the speculative forms are used.
+//
+// Trials that touch one another cannot share a tick: with n_movable / (n_cols + 1) neighbourhoods in the
+// cell, about a third of that many trials can run at once, so small cells take fewer evaluating warps and
+// the smallest stay with the speculative forms, whose rounds they fill.  Measured (FCC, pairs to the 4th
+// shell; ms, half-warp form / here with 8 / 12 / 16 evaluating warps, FP32):
+//   2048 sites, 37 neighbourhoods   3.57 / 2.84 / 2.95 / 3.00     864 sites, 16: 4.87 / 6.1 and more
+//   4000 sites, 73                  4.79 / 2.80 / 2.56 / 2.62
+//   16384 sites, 298                5.36 / 3.20 / 2.69 / 2.61     55296 sites, 1005: 8.63 / 6.44 / 5.26 / 4.86
+bool fit_sched(const cemc_geometry *geo, int rsize, int part, cemc::RunArgs &s) {
+  const cemc::DevGeo &g = geo->g;
+  const int room = g.n_movable / (g.n_cols + 1);
+  if (room < 32) return false;
+  s.warps = room < 64 ? 8 : (room < 128 ? 12 : 16);
+  s.part = part;
+  int exact = 5;
+  while ((1 << exact) < g.n_sites) ++exact;
+  // rows of 512 trials cover the eight or so ticks between a row's fetch and the end of its trial; 256
+  // (which stalls 12 and 16 warps) where the hash would be left with fewer than 2^13 buckets
+  for (int rows = 9; rows >= 8; --rows) {
+    for (int hb = exact; hb >= (rows == 9 ? std::min(exact, 13) : 8); --hb) {
+      s.row_bits = rows;
+      s.ring_bits = rows + 1;  // a mask's 255 trials before the oldest unfinished one stay in the ring
+      s.head_bits = hb;
+      const size_t need = cemc::sched_layout(g, geo->spin.n_cl, geo->spin.n_masks, rsize, 4 * s.warps, s.ring_bits,
+                                             s.row_bits, s.head_bits).total;
+      if (need <= (size_t)geo->max_smem) return true;
+    }
+  }
+  return false;
+}
+
+int run_sched(const cemc_geometry *geo, cemc_run_desc *r, cemc::RunArgs s, void *stream) {
+  const cemc::DevGeo &g = geo->g;
+  const size_t smem = cemc::sched_layout(g, geo->spin.n_cl, geo->spin.n_masks, r->precision == CEMC_PREC_F32 ? 4 : 8,
+                                         4 * s.warps, s.ring_bits, s.row_bits, s.head_bits).total;
+  const uint64_t max_chunk = (uint64_t)1 << 25;  // as the speculative forms; trial numbers of a launch fit 32 bits
+  if (r->n_trials > max_chunk && r->trace_acc)
+    return fail(CEMC_ERR_LIMIT, "traced runs are limited to %llu trials per call", (unsigned long long)max_chunk);
+  for (uint64_t done = 0; done < r->n_trials;) {
+    const uint64_t n = std::min(max_chunk, r->n_trials - done);
+    s.n_trials = n;
+    s.chunk_offset = done;
+    cudaError_t e = cemc::launch_sched(g, s, r->precision, smem, static_cast<cudaStream_t>(stream), geo->spin);
+    if (e != cudaSuccess) return cuda_fail(e, "scheduled Monte Carlo kernel launch");
+    done += n;
+  }
+  r->kernel_used = CEMC_KERNEL_SPIN_QUARTER;
+  return CEMC_OK;
+}
+
+}  // namespace
 
 extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream) {
   if (!geo || !r) return fail(CEMC_ERR_ARG, "null geometry or run descriptor");
@@ -1008,6 +1073,14 @@ extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream
     if (!found && r->cluster != 2) found = fit(1, L, a);
   }
   if (!found) return fail(CEMC_ERR_LIMIT, "shared memory exceeds %zu bytes; use fewer warps", budget);
+  // Scheduled kernel: unconstrained spin flips of the automatic and the quarter-warp form.  It books in the
+  // rounds this launch shape would have had with exact conflict tables, so a shape that would hash them stays.
+  if (geo->spin_ok && geo->spin.qtr_ok && g.table16 && form == cemc::kFormSpin && r->move == CEMC_MOVE_FLIP &&
+      !constrained && r->cluster != 2 && (r->kernel == CEMC_KERNEL_AUTO || r->kernel == CEMC_KERNEL_SPIN_QUARTER) &&
+      (a.gstamp || a.stamp_bits == exact_bits)) {
+    cemc::RunArgs s = a;
+    if (fit_sched(geo, rsize, cemc::round_trials(1, a.warps, a.tpw), s)) return run_sched(geo, r, s, stream);
+  }
   // The table form leaves correlation functions to a full recompute at the end of the call.
   double *rscratch = nullptr;
   if (form == cemc::kFormTable) {

@@ -34,6 +34,8 @@ struct DevGeo {
   int n_slots;     // max ECIs per lane chunk
   int cpad;        // row stride of `table`: n_cols rounded up to a multiple of 4 (16-byte rows)
   const int32_t *table;     // [n_sites * cpad] row-major (trial moves), padding columns repeat column 0
+  const uint16_t *table16;  // the rows in 16 bits, cp16 entries each (n_cols rounded up to a multiple of 8,
+  int cp16;                 // padding repeats column 0), for the scheduled kernel; NULL above 65536 sites
   const int32_t *table_cm;  // [n_cols * n_sites] column-major (full recompute)
   const uint16_t *terms;    // [n_terms * 4]
   const int32_t *lane_term; // [33] chunk boundaries

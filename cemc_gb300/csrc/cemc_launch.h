@@ -37,6 +37,9 @@ struct RunArgs {
   const uint32_t *frozen;
   int max_attempts;
   int accept_first;  // the first trial of the call (chunk offset 0) is accepted whatever its energy change
+  int part;          // scheduled kernel: trials per booking round (the round width of the speculative forms)
+  int row_bits;      // scheduled kernel: log2 of the neighbour-row ring (ring_bits: trials in flight)
+  int head_bits;     // scheduled kernel: log2 of the site-hash size
   int cons;          // 1: the build with the constraint redraw loop and first-move acceptance (one CTA per chain)
 };
 

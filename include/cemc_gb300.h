@@ -201,7 +201,11 @@ typedef struct {
  * for — else the table form when its tables fit, else the generic form.  All
  * give the same decisions for the same stream.  The spin forms evaluate a
  * trial from a bit-packed neighbourhood (popcounts of shell masks, parities of
- * multi-site terms), one trial per warp or one per 16 lanes; the generic form
+ * multi-site terms), one trial per warp, per 16 or per 8 lanes; unconstrained
+ * flips of cells with enough sites, asked for as AUTO or SPIN_QUARTER, run in
+ * the scheduled kernel (trials that do not touch one another in any order; one
+ * per 8 lanes; kernel_used reports SPIN_QUARTER, and `warps` keeps its meaning
+ * only for the rounds the running sums are taken in); the generic form
  * multiplies basis values term by term and keeps the correlation functions up
  * to date trial by trial; the table form looks up one precomputed energy change
  * per cluster geometry (tables built per chain from its ECIs at launch) and
