@@ -18,6 +18,7 @@
 #include <string>
 #include <vector>
 
+#include "cemc_boxcf.h"
 #include "cemc_field.h"
 #include "cemc_kernels.h"
 #include "cemc_sched.h"
@@ -51,6 +52,7 @@ struct cemc_geometry {
   bool spin_ok = false;
   cemc::FieldDev field{};  // tables of the local-field kernel (field_ok)
   bool field_ok = false;
+  cemc::BoxCf box{};  // tables of the bit-plane recompute (box.ok)
   void *dev = nullptr;  // one device allocation holding every table
   size_t dev_bytes = 0;  // its size
   int max_smem = 0;     // opt-in shared memory per block of the current device
@@ -609,6 +611,143 @@ extern "C" int cemc_geometry_create(const cemc_geometry_desc *d, cemc_geometry *
   }
   if (box_off.empty()) box_off.assign(1, 0u);
 
+  // Bit-plane recompute of a periodic box (cemc_boxcf.h): the sub-clusters of every basis site grouped into
+  // orbits under lattice translation, orbits with the same terms into patterns.
+  std::vector<int32_t> bx_job, bx_ent, bx_ent_start, bx_k_start(K + 1, 0), bx_k_count;
+  std::vector<double> bx_k_w, bx_k_const(K, 0.0);
+  int bx_n_counts = 0, bx_hx = 0;
+  const bool bx_pm1 = B == 1 && ((d->bf[0] == 1.0 && d->bf[1] == -1.0) || (d->bf[0] == -1.0 && d->bf[1] == 1.0));
+  bool bx_ok = box_L > 0 && box_L <= cemc::kBoxMaxL && S <= 3;
+  if (bx_ok) {
+    using Point = std::array<int, 4>;                          // x, y, z (mod L), basis site
+    using Term = std::array<int, 5>;                           // ECI, decoration of each point
+    const int L = box_L;
+    std::map<std::vector<int>, std::vector<Term>> geos;        // member columns -> terms (own decoration first)
+    for (int t = 0; t < T; ++t) {
+      std::vector<int> cols;
+      Term tm{d->term_eci[t], d->term_ref[t], 0, 0, 0};
+      for (int j = 0; j < d->term_size[t] - 1; ++j) {
+        cols.push_back(d->term_nb[3 * t + j] / B);
+        tm[2 + j] = d->term_nb[3 * t + j] % B;
+      }
+      geos[cols].push_back(tm);
+    }
+    std::map<std::vector<Point>, std::map<Term, int>> orbits;  // points, the first in cell 0 -> terms and counts
+    for (int b = 0; b < box_nb; ++b)
+      for (const auto &ge : geos) {
+        std::vector<Point> pts{{0, 0, 0, b}};
+        for (int col : ge.first) {
+          const uint32_t o = box_off[(size_t)b * C + col];
+          pts.push_back({(int)(o & 255u) - 128, (int)((o >> 8) & 255u) - 128, (int)((o >> 16) & 255u) - 128, (int)(o >> 24)});
+        }
+        const int n = (int)pts.size();
+        std::vector<Point> best;
+        std::vector<int> order;  // order[i]: position in pts of the i-th canonical point
+        for (int from = 0; from < n; ++from) {
+          std::vector<std::pair<Point, int>> list;
+          for (int i = 0; i < n; ++i) {
+            Point p = pts[i];
+            for (int q = 0; q < 3; ++q) p[q] = ((p[q] - pts[from][q]) % L + L) % L;
+            list.push_back({p, i});
+          }
+          std::sort(list.begin(), list.end());
+          std::vector<Point> key;
+          for (const auto &e : list) key.push_back(e.first);
+          if (best.empty() || key < best) {
+            best = key;
+            order.clear();
+            for (const auto &e : list) order.push_back(e.second);
+          }
+        }
+        auto &terms = orbits[best];
+        for (const Term &tm : ge.second) {
+          Term c{tm[0], 0, 0, 0, 0};
+          if (!bx_pm1)
+            for (int i = 0; i < n; ++i) c[1 + i] = tm[1 + order[i]];
+          terms[c] += 1;
+        }
+      }
+    std::map<std::pair<int, std::map<Term, int>>, int> pats;
+    std::vector<int> pat_first, pat_orbits;                // first counter, orbits
+    std::vector<std::vector<std::array<int, 4>>> pat_ents; // basis site, offsets
+    auto near_l = [&](int v) { return 2 * v > box_L ? v - box_L : v; };
+    auto pack_point = [&](const Point &p) {
+      const int x = near_l(p[0]), y = near_l(p[1]);
+      bx_hx = std::max(bx_hx, std::abs(x));
+      return (int)((uint32_t)(x + 128) | ((uint32_t)(y + 128) << 8) | ((uint32_t)p[2] << 16) | ((uint32_t)p[3] << 24));
+    };
+    for (const auto &ob : orbits) {
+      const int n = (int)ob.first.size();
+      const auto key = std::make_pair(n, ob.second);
+      auto it = pats.find(key);
+      if (it == pats.end()) {
+        it = pats.emplace(key, (int)pats.size()).first;
+        int tuples = 1;
+        for (int i = 0; i < n && !bx_pm1; ++i) tuples *= S;
+        pat_first.push_back(bx_n_counts);
+        bx_n_counts += tuples;
+        pat_orbits.push_back(0);
+        pat_ents.push_back({});
+      }
+      pat_orbits[it->second] += 1;
+      std::array<int, 4> e{ob.first[0][3], 0, 0, 0};
+      for (int i = 1; i < n; ++i) e[i] = pack_point(ob.first[i]);
+      pat_ents[it->second].push_back(e);
+    }
+    // jobs: the orbits of a pattern, by basis site of their first point, kBoxJob of each at a time
+    bx_ent_start.assign(1, 0);
+    for (const auto &pt : pats) {
+      std::vector<std::vector<std::array<int, 4>>> by_b(box_nb);
+      size_t most = 0;
+      for (const auto &e : pat_ents[pt.second]) by_b[e[0]].push_back(e);
+      for (const auto &v : by_b) most = std::max(most, v.size());
+      for (size_t at = 0; at < most; at += cemc::kBoxJob) {
+        bx_job.insert(bx_job.end(), {pt.first.first, pat_first[pt.second]});
+        for (const auto &v : by_b) {
+          for (size_t i = at; i < std::min(v.size(), at + cemc::kBoxJob); ++i)
+            bx_ent.insert(bx_ent.end(), {v[i][1], v[i][2], v[i][3], 0});
+          bx_ent_start.push_back((int32_t)(bx_ent.size() / 4));
+        }
+      }
+    }
+    // each ECI's sum over all sites as a weighted sum of counters
+    const double cells = (double)(N / box_nb);
+    std::vector<std::map<int, double>> w(K);
+    for (const auto &pt : pats) {
+      const int n = pt.first.first, id = pt.second, c0 = pat_first[id];
+      for (const auto &tm : pt.first.second) {
+        const int k = tm.first[0];
+        const double mult = (double)tm.second;
+        if (bx_pm1) {
+          w[k][c0] -= 2.0 * mult;
+          bx_k_const[k] += mult * cells * pat_orbits[id];
+          continue;
+        }
+        int tuples = 1;
+        for (int i = 0; i < n; ++i) tuples *= S;
+        for (int q = 0; q < tuples; ++q) {
+          double v = mult;
+          for (int i = 0, r = q; i < n; ++i, r /= S) v *= d->bf[tm.first[1 + i] * S + r % S];
+          w[k][c0 + q] += v;
+        }
+      }
+    }
+    for (int k = 0; k < K; ++k) {
+      for (const auto &e : w[k]) {
+        bx_k_count.push_back(e.first);
+        bx_k_w.push_back(e.second);
+      }
+      bx_k_start[k + 1] = (int32_t)bx_k_count.size();
+    }
+    bx_ok = !bx_job.empty() && bx_n_counts <= cemc::kBoxMaxCounts;
+  }
+  const int bx_n_jobs = (int)(bx_job.size() / 2), bx_n_ents = (int)(bx_ent.size() / 4);
+  if (bx_job.empty()) bx_job.assign(2, 0);
+  if (bx_ent.empty()) bx_ent.assign(4, 0);
+  if (bx_ent_start.empty()) bx_ent_start.assign(1, 0);
+  if (bx_k_count.empty()) bx_k_count.assign(1, 0);
+  if (bx_k_w.empty()) bx_k_w.assign(1, 0.0);
+
   // One device allocation for all tables.
   struct Part {
     const void *src;
@@ -650,6 +789,13 @@ extern "C" int cemc_geometry_create(const cemc_geometry_desc *d, cemc_geometry *
       {qtr_lane_term.data(), 9 * 4, 0},
       {qtr_lane_first.data(), 8 * 4, 0},
       {table16.data(), table16.size() * 2, 0},
+      {bx_job.data(), bx_job.size() * 4, 0},
+      {bx_ent.data(), bx_ent.size() * 4, 0},
+      {bx_ent_start.data(), bx_ent_start.size() * 4, 0},
+      {bx_k_start.data(), bx_k_start.size() * 4, 0},
+      {bx_k_count.data(), bx_k_count.size() * 4, 0},
+      {bx_k_w.data(), bx_k_w.size() * 8, 0},
+      {bx_k_const.data(), bx_k_const.size() * 8, 0},
   };
   size_t total = 0;
   for (auto &p : parts) {
@@ -723,6 +869,19 @@ extern "C" int cemc_geometry_create(const cemc_geometry_desc *d, cemc_geometry *
     if (d->bf[0] == 1.0 && d->bf[1] == -1.0) g.pm1_minus = 1;
     else if (d->bf[0] == -1.0 && d->bf[1] == 1.0) g.pm1_minus = 0;
   }
+  geo->box.ok = bx_ok ? 1 : 0;
+  geo->box.pm1 = bx_pm1 ? 1 : 0;
+  geo->box.n_jobs = bx_n_jobs;
+  geo->box.n_ents = bx_n_ents;
+  geo->box.n_counts = bx_n_counts;
+  geo->box.hx = bx_hx;
+  geo->box.job = reinterpret_cast<const int2 *>(base + parts[40].off);
+  geo->box.ent = reinterpret_cast<const int4 *>(base + parts[41].off);
+  geo->box.ent_start = reinterpret_cast<const int32_t *>(base + parts[42].off);
+  geo->box.k_start = reinterpret_cast<const int32_t *>(base + parts[43].off);
+  geo->box.k_count = reinterpret_cast<const int32_t *>(base + parts[44].off);
+  geo->box.k_w = reinterpret_cast<const double *>(base + parts[45].off);
+  geo->box.k_const = reinterpret_cast<const double *>(base + parts[46].off);
   geo->spin_ok = spin_ok;
   geo->spin.n_cl = spin_ok ? (int)spin_eci.size() : 0;
   geo->spin.n_masks = spin_ok ? n_masks : 0;
@@ -780,6 +939,16 @@ extern "C" size_t cemc_stamp_words(const cemc_geometry *geo, int32_t n_chains) {
 }
 
 namespace {
+
+// Full recompute: by bit planes in a periodic box, else term by term through the neighbour table.
+cudaError_t recompute(const cemc_geometry *geo, int n_chains, const int8_t *occ, const double *eci, double *cf,
+                      double *energy, double *scratch, void *stream) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  size_t smem = 0;
+  const int ctas = cemc::boxcf_ctas(geo->g, geo->box, n_chains, geo->n_sms, (size_t)geo->max_smem, &smem);
+  if (ctas) return cemc::launch_boxcf(geo->g, geo->box, n_chains, ctas, smem, occ, eci, cf, energy, st);
+  return cemc::launch_recompute(geo->g, n_chains, occ, eci, cf, energy, scratch, st);
+}
 
 // Shape of the scheduled kernel for this geometry, or false where the speculative forms are used.
 //
@@ -1115,8 +1284,7 @@ extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream
                   : (form == cemc::kFormGeneric || form == cemc::kFormRecycle) ? CEMC_KERNEL_GENERIC
                   : (a.tpw == 4 ? CEMC_KERNEL_SPIN_QUARTER : a.tpw == 2 ? CEMC_KERNEL_SPIN_HALFWARP : CEMC_KERNEL_SPIN);
   if (form == cemc::kFormTable) {
-    cudaError_t e = cemc::launch_recompute(g, r->n_chains, r->occ, r->eci, r->cf, r->energy, rscratch,
-                                           static_cast<cudaStream_t>(stream));
+    cudaError_t e = recompute(geo, r->n_chains, r->occ, r->eci, r->cf, r->energy, rscratch, stream);
     if (e != cudaSuccess) return cuda_fail(e, "recompute after the table kernel");
   }
   return CEMC_OK;
@@ -1132,8 +1300,7 @@ extern "C" int cemc_recompute(const cemc_geometry *geo, int32_t n_chains, const 
   if (!geo || n_chains <= 0 || !occ || !eci || !cf || !energy || !scratch)
     return fail(CEMC_ERR_ARG, "bad recompute arguments");
   if (n_chains > 65535) return fail(CEMC_ERR_LIMIT, "too many chains in one recompute");
-  cudaError_t e = cemc::launch_recompute(geo->g, n_chains, occ, eci, cf, energy, scratch,
-                                         static_cast<cudaStream_t>(stream));
+  cudaError_t e = recompute(geo, n_chains, occ, eci, cf, energy, scratch, stream);
   if (e != cudaSuccess) return cuda_fail(e, "recompute kernel launch");
   return CEMC_OK;
 }
@@ -1154,8 +1321,7 @@ extern "C" int cemc_recompute_noalloc(const cemc_geometry *geo, int32_t n_chains
   if (!scratch) return cuda_fail(err, "cudaGetSymbolAddress(recompute_noalloc scratch)");
   // Each scratch entry the second kernel reads is written by the first kernel
   // of the same call, so nothing has to be cleared between calls.
-  cudaError_t e = cemc::launch_recompute(geo->g, n_chains, occ, eci, cf, energy, scratch,
-                                         static_cast<cudaStream_t>(stream));
+  cudaError_t e = recompute(geo, n_chains, occ, eci, cf, energy, scratch, stream);
   if (e != cudaSuccess) return cuda_fail(e, "recompute_noalloc kernel launch");
   return CEMC_OK;
 }
