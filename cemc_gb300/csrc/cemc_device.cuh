@@ -222,6 +222,20 @@ __device__ __forceinline__ int metropolis(R de, uint32_t ua, uint32_t ub, double
   return cemc_u01_53(ua, ub) <= exp(-(double)de / kT);
 }
 
+// The same test of an energy change held as an integer multiple of a quantum (`de` its FP64 value): x =
+// dE/kT is its float conversion times the float quantum / kT, two roundings more than above.
+template <typename R>
+__device__ __forceinline__ int metropolis_fx(long long de_fx, R de, uint32_t ua, uint32_t ub, double kT, float q_kT) {
+  if (de_fx < 0) return 1;
+  const float x = (float)de_fx * q_kT;
+  const float uf = (float)ua * 2.3283064e-10f;  // a * 2^-32
+  const float y = __logf(uf) + x;
+  const float margin = 1e-4f + 1e-6f * x + 1e-8f / uf;  // uf == 0 gives an infinite margin
+  if (y < -margin) return 1;
+  if (y > margin) return 0;
+  return cemc_u01_53(ua, ub) <= exp(-(double)de / kT);
+}
+
 // The same test with the uniform's parts precomputed (by the fetcher, off the
 // evaluating warps' path): lnu = __logf(u) and mu = 1e-4 + 1e-8 / u for
 // u = ua * 2^-32.  The margin can differ from metropolis()'s in its last bit,

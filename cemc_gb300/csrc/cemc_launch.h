@@ -79,7 +79,7 @@ struct McLayout {
   size_t rec, rec_stride, rec_sa, rec_sb, rec_de, rec_ds, rec_acc, rec_la, rec_lb, rec_A, rec_B;
   size_t drow;  // [2][warps * tpw][n_eci] correlation-function changes of this CTA's trials
   size_t cfp;   // spin form: per-lane sums of booked change rows [2][n_eci][32] (int32)
-  size_t ftab, geos;  // table form
+  size_t ftab, geos, sfx;  // table form
   size_t draws, rows;
   size_t warp0, warp_stride, warp_part;
   size_t occ, trk, stamp;
@@ -165,6 +165,8 @@ __host__ __device__ inline McLayout mc_layout(const DevGeo &g, int warps, int mo
   if (table) o = align16(o + (size_t)rsize * g.tab_len);
   L.geos = o;
   if (table) o = align16(o + 16 * (size_t)g.n_geo);
+  L.sfx = o;  // FP64: singlet energies per (old, new) species in fixed point
+  if (table && rsize == 8) o = align16(o + 8 * (size_t)(g.n_sym * g.n_sym));
   const size_t ring = (size_t)1 << ring_bits;
   L.draws = o;
   o = align16(o + sizeof(Draw) * ring);

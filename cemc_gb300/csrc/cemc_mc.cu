@@ -166,19 +166,39 @@ __device__ __forceinline__ void table_gather(const DevGeo &g, const int8_t *occ,
 // Energy change of one flip (or, TWO, of a swap's two flips) from the pattern
 // tables: one lookup per cluster geometry, F[off + on * S^m + s1 + S s2 + S^2 s3]
 // with on = old * S + new and the member species s_j of the geometry's columns.
-// Geometries [lo, hi) are those of the changed site's translation group.
-template <typename R, bool TWO>
-__device__ __forceinline__ R table_de(const DevGeo &g, const uint4 *geos, const R *F, const int8_t *spa,
-                                      const int8_t *spb, int on_a, int on_b, int lo, int hi, int lane) {
-  const int S = g.n_sym, S2 = S * S;
-  R sum = (R)0;
+// Geometries [lo, hi) are those of the changed site's translation group, packed as
+// {c1 | c2 << 8 | c3 << 16, off, S^m, 0}.  Lane l adds geometries lo + l, lo + l + 32, .. in this order, then a butterfly.
+//
+// T is the entries' type: float, double, or int64 fixed-point (FP64 launches; see fixed_point_scale()).
+// (Four lookups in flight at a time, with the geometries in shared memory or in registers, measured slower:
+// ladder 34.1 -> 35.1 and 43 ms, the loop is bound by its shared-memory wavefronts and instructions.)
+template <typename T, bool TWO>
+__device__ __forceinline__ T table_sum(int S, const uint4 *geos, const T *F, const int8_t *spa, const int8_t *spb,
+                                       int on_a, int on_b, int lo, int hi, int lane) {
+  const int S2 = S * S;
+  T sum = (T)0;
   for (int i = lo + lane; i < hi; i += 32) {
     const uint4 e = geos[i];
     const int c1 = e.x & 0xff, c2 = (e.x >> 8) & 0xff, c3 = (e.x >> 16) & 0xff;
     sum += F[e.y + on_a * e.z + spa[c1] + S * spa[c2] + S2 * spa[c3]];
     if (TWO) sum += F[e.y + on_b * e.z + spb[c1] + S * spb[c2] + S2 * spb[c3]];
   }
-  return warp_sum(sum);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
+  return sum;
+}
+
+// FP64 launches hold the table entries as int64 multiples of 2^-k: this part's FP64 pipe issues one warp
+// instruction in 16 cycles per SM, so 30 additions in each of 16 warps cost more than the rest of a round,
+// while 64-bit integer additions are two instructions on the wide pipe, and exact.  k is as large as sums
+// of 2 n entries of magnitude `most` allow (|sum| < 2^61), i.e. the quantum is at most 2^-60 n most: for 458
+// geometries of 0.1 eV 4e-17 eV, the spacing of FP64 numbers near 0.3 eV.  0: not representable (an ECI that
+// is infinite or NaN), the entries stay FP64.
+__device__ __forceinline__ double fixed_point_scale(double most, int n) {
+  const double bound = most * 2.0 * (double)(n + 1);
+  if (!(bound < 1e300)) return 0.0;
+  if (!(bound > 1e-200)) return 1.0;
+  return ldexp(1.0, 60 - ilogb(bound));
 }
 
 // ---- thread-block cluster pairs ---------------------------------------------
@@ -310,6 +330,9 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
   int8_t *sp_b = sp_a + align16((size_t)g.n_cols + 1);
   R *ftab = reinterpret_cast<R *>(smem + L.ftab);
   uint4 *geos_s = reinterpret_cast<uint4 *>(smem + L.geos);
+  constexpr bool FX = TAB && sizeof(R) == 8;  // table entries in fixed point, if they can be
+  long long *ftab_fx = reinterpret_cast<long long *>(smem + L.ftab);
+  long long *sfx_s = reinterpret_cast<long long *>(smem + L.sfx);  // [old * S + new] energy of the singlets' change
   R *vb = va + g.vals_len;
   R *part = reinterpret_cast<R *>(wbase + L.warp_part);
 
@@ -738,6 +761,33 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
     cluster_barrier();  // the peer's tables are initialised before any remote store
   else
     __syncthreads();
+  double fx_scale = 0.0, fx_inv = 0.0;  // table entries are multiples of fx_inv (0: they are FP64)
+  float fx_kT = 0.f;
+  if constexpr (FX) {
+    const int S = g.n_sym;
+    double most = 0.0;  // every warp finds it for itself
+    for (int i = lane; i < g.tab_len; i += 32) most = fmax(most, isnan(ftab[i]) ? HUGE_VAL : fabs((double)ftab[i]));
+    for (int i = lane; i < n_eci; i += 32)
+      if (kind_s[i] == 1)
+        for (int s = 0; s < S * S; ++s)
+          most = fmax(most, isnan(eci_s[i]) ? HUGE_VAL
+                                            : fabs(eci_s[i] * (bf_s[dec_s[i] * S + s % S] - bf_s[dec_s[i] * S + s / S])));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) most = fmax(most, __shfl_xor_sync(kFull, most, o));
+    fx_scale = fixed_point_scale(most, g.n_geo + CEMC_MAX_BF);
+    __syncthreads();
+    if (fx_scale != 0.0) {
+      fx_inv = 1.0 / fx_scale;
+      fx_kT = (float)(fx_inv / kT);
+      for (int i = tid; i < g.tab_len; i += blockDim.x) ftab_fx[i] = __double2ll_rn((double)ftab[i] * fx_scale);
+      for (int s = tid; s < S * S; s += blockDim.x) {
+        double v = 0.0;
+        for (int b = 0; b < g.n_bf; ++b)
+          if (g.singlet_eci[b] >= 0) v += coef_s[g.singlet_eci[b]] * (bf_s[b * S + s % S] - bf_s[b * S + s / S]);
+        sfx_s[s] = __double2ll_rn(v * fx_scale);
+      }
+    }
+  }
   if (misc[1] != 0) {  // same verdict in both CTAs of a pair: it depends on the chain's inputs only
     if (tid == 0 && rank == 0 && a.status) a.status[chain] = misc[1];
     return;
@@ -1078,21 +1128,35 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
               gb = g.site_group[sb];
             }
           }
+          long long de_fx = 0;  // the energy change in units of fx_inv
           if constexpr (TAB) {
             __syncwarp();
             const int S = g.n_sym;
-            if (!SWAP) {
-              de = table_de<R, false>(g, geos_s, ftab, sp_a, sp_b, old_a * S + na, 0, gstart_s[ga], gstart_s[ga + 1],
-                                      lane);
-              for (int b = 0; b < g.n_bf; ++b)
-                if (g.singlet_eci[b] >= 0)
-                  de += coef_s[g.singlet_eci[b]] * (bf_s[b * S + na] - bf_s[b * S + old_a]);
-            } else if (ga == gb) {
-              de = table_de<R, true>(g, geos_s, ftab, sp_a, sp_b, A_ * S + B_, B_ * S + A_, gstart_s[ga],
-                                     gstart_s[ga + 1], lane);
+            // energy change by the tables of type T (the swap's two sites in one pass, unless their groups differ)
+            auto change = [&](auto *F) {
+              if constexpr (!SWAP)
+                return table_sum<std::remove_pointer_t<decltype(F)>, false>(S, geos_s, F, sp_a, sp_a, old_a * S + na, 0,
+                                                                           gstart_s[ga], gstart_s[ga + 1], lane);
+              else if (ga == gb)
+                return table_sum<std::remove_pointer_t<decltype(F)>, true>(S, geos_s, F, sp_a, sp_b, A_ * S + B_,
+                                                                          B_ * S + A_, gstart_s[ga], gstart_s[ga + 1],
+                                                                          lane);
+              else
+                return table_sum<std::remove_pointer_t<decltype(F)>, false>(S, geos_s, F, sp_a, sp_a, A_ * S + B_, 0,
+                                                                           gstart_s[ga], gstart_s[ga + 1], lane) +
+                       table_sum<std::remove_pointer_t<decltype(F)>, false>(S, geos_s, F, sp_b, sp_b, B_ * S + A_, 0,
+                                                                           gstart_s[gb], gstart_s[gb + 1], lane);
+            };
+            if (FX && fx_scale != 0.0) {
+              de_fx = change(ftab_fx);
+              if (!SWAP) de_fx += sfx_s[old_a * S + na];
+              de = (R)((double)de_fx * fx_inv);
             } else {
-              de = table_de<R, false>(g, geos_s, ftab, sp_a, sp_a, A_ * S + B_, 0, gstart_s[ga], gstart_s[ga + 1], lane) +
-                   table_de<R, false>(g, geos_s, ftab, sp_b, sp_b, B_ * S + A_, 0, gstart_s[gb], gstart_s[gb + 1], lane);
+              de = change(ftab);
+              if (!SWAP)
+                for (int b = 0; b < g.n_bf; ++b)
+                  if (g.singlet_eci[b] >= 0)
+                    de += coef_s[g.singlet_eci[b]] * (bf_s[b * S + na] - bf_s[b * S + old_a]);
             }
             __syncwarp();
           } else if constexpr (!SPIN) {
@@ -1148,7 +1212,10 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
             if constexpr (RECYCLE)
               acc = no_move ? 0 : (first ? 1 : barker<R>(de, ua, ub, kT));
             else
-              acc = no_move ? 0 : (first ? 1 : metropolis<R>(de, ua, ub, kT, inv_kT));
+              acc = no_move ? 0
+                            : (first ? 1
+                                     : (FX && fx_scale != 0.0 ? metropolis_fx(de_fx, de, ua, ub, kT, fx_kT)
+                                                              : metropolis<R>(de, ua, ub, kT, inv_kT)));
             if (CONS && no_move) put(&misc[3], 1);  // reported in the status at the end of the launch
             put(&r_sa[gidx], (int32_t)sa);
             put(&r_sb[gidx], (int32_t)(SWAP ? sb : na));
