@@ -22,6 +22,7 @@
 #include "cemc_field.h"
 #include "cemc_kernels.h"
 #include "cemc_sched.h"
+#include "cemc_schedt.h"
 #include "cemc_spin.h"
 
 namespace {
@@ -982,6 +983,39 @@ bool fit_sched(const cemc_geometry *geo, int rsize, int part, cemc::RunArgs &s) 
   return false;
 }
 
+// Shape of the scheduled table kernel, or false where the speculative form is used.
+//
+// `room` is the number of neighbourhoods of a move's sites in the cell; about a third of it can run at once.
+// Measured (ms; speculative form in the default or its best explicit width / here with 8 / 16 / 24 trials a
+// tick; FP32 unless said):
+//   swaps   78 columns: 1372 sites, room 4   4.07 / 4.92 / 5.83 / 7.10     4000, 12   5.93 / 4.44 / 4.90 / 6.17
+//                       16384, 51            4.30 / 2.83 / 2.39 / 2.64     55296, 174 6.03 / 5.55 / 4.27 / 4.24
+//           86 columns: 131072, 376         10.25 / 15.9 / 10.0 / 9.08
+//           18 columns: 1000, 13             2.13 / 2.39 / 2.60            3528, 46   2.71 / 2.58 / 2.22
+//   flips   78 columns: 4000, 50             3.53 / 3.56 / 2.97 (FP64 3.83 / 4.32 / 4.08)
+//           18 columns: 1000, 52             0.96 / 1.22 / 1.05            3528, 185  1.24 / 1.77 / 1.25
+// A flip's rows and draws are as cheap ahead in the speculative form, so flips gain only where the evaluation
+// is long, and in FP64 the booking of their singlets (FP64 scans) takes what they gain.
+bool fit_tick(const cemc_geometry *geo, int precision, int move, int part, cemc::RunArgs &s) {
+  const cemc::DevGeo &g = geo->g;
+  const bool swap = move == CEMC_MOVE_SWAP;
+  const int room = g.n_movable / ((swap ? 4 : 1) * (g.n_cols + 1));
+  const bool wide = g.n_cols >= 48;
+  if (part > 32 || (swap ? room < (wide ? 10 : 40) : (precision != CEMC_PREC_F32 || !wide || room < 40))) return false;
+  s.part = part;
+  s.warps = swap && room < 20 ? 8 : (swap && room >= 150 ? cemc::kTickCap : cemc::kTickWarps);
+  int exact = 5;
+  while ((1 << exact) < g.n_sites) ++exact;
+  for (int rb = 7; rb >= 6; --rb)
+    for (int hb = std::min(exact, 14); hb >= std::min(exact, 11); --hb) {
+      s.row_bits = rb;
+      s.head_bits = hb;
+      if (cemc::tick_layout(g, swap, precision == CEMC_PREC_F32 ? 4 : 8, rb, hb).total <= (size_t)geo->max_smem)
+        return true;
+    }
+  return false;
+}
+
 int run_sched(const cemc_geometry *geo, cemc_run_desc *r, cemc::RunArgs s, void *stream) {
   const cemc::DevGeo &g = geo->g;
   const size_t smem = cemc::sched_layout(g, geo->spin.n_cl, geo->spin.n_masks, r->precision == CEMC_PREC_F32 ? 4 : 8,
@@ -1271,8 +1305,23 @@ extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream
   const uint64_t max_chunk = (uint64_t)1 << 25;
   if (r->n_trials > max_chunk && r->trace_acc)
     return fail(CEMC_ERR_LIMIT, "traced runs are limited to %llu trials per call", (unsigned long long)max_chunk);
+  // Scheduled table kernel: unconstrained moves of the table form, booked in the rounds this launch shape
+  // would have had with exact conflict tables (a shape that would hash them stays).
+  cemc::RunArgs tick = a;
+  size_t tick_smem = 0;
+  if (form == cemc::kFormTable && !constrained && (a.gstamp || a.stamp_bits == exact_bits) &&
+      fit_tick(geo, r->precision, r->move, cemc::round_trials(a.cl, a.warps, a.tpw), tick))
+    tick_smem = cemc::tick_layout(g, is_swap, rsize, tick.row_bits, tick.head_bits).total;
   for (uint64_t done = 0; done < r->n_trials;) {
     const uint64_t n = std::min(max_chunk, r->n_trials - done);
+    if (tick_smem) {
+      tick.n_trials = n;
+      tick.chunk_offset = done;
+      cudaError_t e = cemc::launch_tick(g, tick, r->move, r->precision, tick_smem, static_cast<cudaStream_t>(stream));
+      if (e != cudaSuccess) return cuda_fail(e, "scheduled table kernel launch");
+      done += n;
+      continue;
+    }
     a.n_trials = n;
     a.chunk_offset = done;
     cudaError_t e = cemc::launch_mc(g, a, r->move, r->precision, L.total, static_cast<cudaStream_t>(stream), form,

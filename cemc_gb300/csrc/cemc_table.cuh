@@ -1,0 +1,89 @@
+// Table form of the trial energy change, shared by the speculative (cemc_mc.cu) and the scheduled
+// (cemc_schedt.cu) kernels.
+#pragma once
+#include "cemc_device.cuh"
+
+namespace cemc {
+
+// Entry `idx` of a chain's pattern tables, F(old, new, member species), in FP64.
+__device__ inline double table_entry(const DevGeo &g, const double *eci, int idx) {
+  const int S = g.n_sym;
+  int p = 0;
+  while (p + 1 < g.n_pat && g.pat_info[p + 1].y <= idx) ++p;
+  const int4 pi = g.pat_info[p];
+  int stride = 1;
+  for (int j = 0; j < pi.x; ++j) stride *= S;
+  const int li = idx - pi.y, on = li / stride, tup = li - on * stride;
+  const int old_s = on / S, new_s = on - old_s * S;
+  double v = 0.0;
+  for (int t = pi.z; t < pi.w; ++t) {
+    const int pk = g.pat_terms[t];
+    const int k = pk & 0xff, dr = (pk >> 8) & 15;
+    double prod = g.bf[dr * S + new_s] - g.bf[dr * S + old_s];
+    int tt = tup;
+    for (int j = 0; j < pi.x; ++j) {
+      const int sj = tt % S;
+      tt /= S;
+      prod *= g.bf[((pk >> (12 + 4 * j)) & 15) * S + sj];
+    }
+    v += eci[k] * (double)g.n_sites * g.eci_w[k] * prod;
+  }
+  return v;
+}
+
+// Largest magnitude of a chain's table entries and singlet energies (one warp; NaN counts as infinite).
+template <typename R>
+__device__ inline double table_most(const DevGeo &g, const R *ftab, const double *eci, int lane) {
+  const int S = g.n_sym;
+  double most = 0.0;
+  for (int i = lane; i < g.tab_len; i += 32) most = fmax(most, isnan((double)ftab[i]) ? HUGE_VAL : fabs((double)ftab[i]));
+  for (int i = lane; i < g.n_eci; i += 32)
+    if (g.eci_kind[i] == 1) {
+      const double *bf = g.bf + g.eci_dec[i] * S;
+      for (int s = 0; s < S * S; ++s)
+        most = fmax(most, isnan(eci[i]) ? HUGE_VAL : fabs(eci[i] * (bf[s % S] - bf[s / S])));
+    }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) most = fmax(most, __shfl_xor_sync(kFull, most, o));
+  return most;
+}
+
+// Energy change of one flip (or, TWO, of a swap's two flips) from the pattern
+// tables: one lookup per cluster geometry, F[off + on * S^m + s1 + S s2 + S^2 s3]
+// with on = old * S + new and the member species s_j of the geometry's columns.
+// Geometries [lo, hi) are those of the changed site's translation group, packed as
+// {c1 | c2 << 8 | c3 << 16, off, S^m, 0}.  Lane l adds geometries lo + l, lo + l + 32, .. in this order, then a butterfly.
+//
+// T is the entries' type: float, double, or int64 fixed-point (FP64 launches; see fixed_point_scale()).
+// (Four lookups in flight at a time, with the geometries in shared memory or in registers, measured slower:
+// ladder 34.1 -> 35.1 and 43 ms, the loop is bound by its shared-memory wavefronts and instructions.)
+template <typename T, bool TWO>
+__device__ __forceinline__ T table_sum(int S, const uint4 *geos, const T *F, const int8_t *spa, const int8_t *spb,
+                                       int on_a, int on_b, int lo, int hi, int lane) {
+  const int S2 = S * S;
+  T sum = (T)0;
+  for (int i = lo + lane; i < hi; i += 32) {
+    const uint4 e = geos[i];
+    const int c1 = e.x & 0xff, c2 = (e.x >> 8) & 0xff, c3 = (e.x >> 16) & 0xff;
+    sum += F[e.y + on_a * e.z + spa[c1] + S * spa[c2] + S2 * spa[c3]];
+    if (TWO) sum += F[e.y + on_b * e.z + spb[c1] + S * spb[c2] + S2 * spb[c3]];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
+  return sum;
+}
+
+// FP64 launches hold the table entries as int64 multiples of 2^-k: this part's FP64 pipe issues one warp
+// instruction in 16 cycles per SM, so 30 additions in each of 16 warps cost more than the rest of a round,
+// while 64-bit integer additions are two instructions on the wide pipe, and exact.  k is as large as sums
+// of 2 n entries of magnitude `most` allow (|sum| < 2^61), i.e. the quantum is at most 2^-60 n most: for 458
+// geometries of 0.1 eV 4e-17 eV, the spacing of FP64 numbers near 0.3 eV.  0: not representable (an ECI that
+// is infinite or NaN), the entries stay FP64.
+__device__ __forceinline__ double fixed_point_scale(double most, int n) {
+  const double bound = most * 2.0 * (double)(n + 1);
+  if (!(bound < 1e300)) return 0.0;
+  if (!(bound > 1e-200)) return 1.0;
+  return ldexp(1.0, 60 - ilogb(bound));
+}
+
+}  // namespace cemc
