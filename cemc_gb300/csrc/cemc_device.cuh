@@ -252,10 +252,35 @@ __device__ __forceinline__ int metropolis_pre(R de, float lnu, float mu, const u
   if (y > margin) return 0;
   return cemc_u01_53(uw[0], uw[1]) <= exp(-(double)de / kT);
 }
+// metropolis_pre() of an energy change held as an integer multiple of a quantum (see metropolis_fx).
+template <typename R>
+__device__ __forceinline__ int metropolis_pre_fx(long long de_fx, R de, float lnu, float mu, const uint32_t *uw,
+                                                 double kT, float q_kT) {
+  if (de_fx < 0) return 1;
+  const float x = (float)de_fx * q_kT;
+  const float y = lnu + x;
+  const float margin = mu + 1e-6f * x;  // u == 0 gives an infinite margin
+  if (y < -margin) return 1;
+  if (y > margin) return 0;
+  return cemc_u01_53(uw[0], uw[1]) <= exp(-(double)de / kT);
+}
 __device__ __forceinline__ void metropolis_parts(uint32_t ua, float &lnu, float &mu) {
   const float uf = (float)ua * 2.3283064e-10f;  // a * 2^-32
   lnu = __logf(uf);
   mu = 1e-4f + 1e-8f / uf;
+}
+
+// FP64 launches hold table entries and ECI coefficients as int64 multiples of 2^-k: this part's FP64 pipe
+// issues one warp instruction in 16 cycles per SM, so the additions of an energy change in each of 16 warps
+// cost more than the rest of a round, while 64-bit integer additions are two instructions on the wide pipe,
+// and exact.  k is as large as sums of 2 n entries of magnitude `most` allow (|sum| < 2^61), i.e. the quantum
+// is at most 2^-60 n most: for 458 geometries of 0.1 eV 4e-17 eV, the spacing of FP64 numbers near 0.3 eV.
+// 0: not representable (an ECI that is infinite or NaN), everything stays FP64.
+__device__ __forceinline__ double fixed_point_scale(double most, int n) {
+  const double bound = most * 2.0 * (double)(n + 1);
+  if (!(bound < 1e300)) return 0.0;
+  if (!(bound > 1e-200)) return 1.0;
+  return ldexp(1.0, 60 - ilogb(bound));
 }
 
 // Two-state acceptance of waste recycling (Frenkel, PNAS 101, 17571 (2004);

@@ -736,6 +736,8 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
   // spin path: lane k of every evaluating warp holds cluster ECI k and its coefficient
   SpinEci sp_e{};
   R sp_coef = (R)0;
+  long long sp_cfx = 0, sing_fx = 0;  // FP64: the coefficients in units of fx_inv
+  constexpr bool SFX = SPIN && sizeof(R) == 8;
   unsigned sp_multi = 0;  // cluster ECIs with multi-site terms
   // Flips at one or two trials per warp: the odd-term counts of all multi-site ECIs by one
   // packed butterfly (odd_counts_packed) when each has at most 255 terms and their 8-bit
@@ -752,6 +754,19 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
     if (el < sd.n_cl) {
       sp_e = sp_eci[el];
       sp_coef = coef_s[sp_e.eci];
+    }
+    if constexpr (sizeof(R) == 8) {
+      // |P| is at most the ECI's terms (swaps: twice), the spin change 2
+      const double own = lane < 32 / TPW ? (SWAP ? 4.0 : 2.0) * fabs((double)sp_coef) * (double)(sp_e.n_pairs + sp_e.n_multi)
+                                         : 0.0;
+      const double sing = sd.singlet_eci >= 0 && !SWAP ? (double)coef_s[sd.singlet_eci] : 0.0;
+      fx_scale = fixed_point_scale(warp_sum(own) + 2.0 * fabs(sing), 0);
+      if (fx_scale != 0.0) {
+        fx_inv = 1.0 / fx_scale;
+        fx_kT = (float)(fx_inv / kT);
+        sp_cfx = __double2ll_rn((double)sp_coef * fx_scale);
+        sing_fx = __double2ll_rn(sing * fx_scale);
+      }
     }
     sp_multi = __ballot_sync(kFull, el < sd.n_cl && sp_e.n_multi > 0);
     if constexpr (TPW >= 2) sp_multi &= (1u << (32 / TPW)) - 1u;
@@ -921,22 +936,34 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
             P = sp_e.n_pairs - 2 * (__popc(wl & sp_e.pair_lo) + __popc(wh & sp_e.pair_hi)) + sp_e.n_multi - 2 * my_odd;
             if (has) Dh[sp_e.eci] = delta * P;
           }
-          R sum = sp_coef * (R)P;
+          R de;
+          long long de_fx = 0;
+          if (SFX && fx_scale != 0.0) {
+            if (sd.singlet_eci >= 0 && hl == 0 && has) Dh[sd.singlet_eci] = delta;
+            long long sum = sp_cfx * (long long)P;
 #pragma unroll
-          for (int o = LW / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
-          if (sd.singlet_eci >= 0) {
-            if (hl == 0 && has) Dh[sd.singlet_eci] = delta;
-            sum += coef_s[sd.singlet_eci];
+            for (int o = LW / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
+            de_fx = (sum + sing_fx) * (long long)delta;
+            de = (R)((double)de_fx * fx_inv);
+          } else {
+            R sum = sp_coef * (R)P;
+#pragma unroll
+            for (int o = LW / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
+            if (sd.singlet_eci >= 0) {
+              if (hl == 0 && has) Dh[sd.singlet_eci] = delta;
+              sum += coef_s[sd.singlet_eci];
+            }
+            de = (R)delta * sum;
           }
-          const R de = (R)delta * sum;
           int acc = 0;
           if (hl == 0 && has) {
-            acc = metropolis_pre<R>(de, lnu, mu, &draws[slot].x0, kT, inv_kT);
+            acc = SFX && fx_scale != 0.0 ? metropolis_pre_fx(de_fx, de, lnu, mu, &draws[slot].x0, kT, fx_kT)
+                                         : metropolis_pre<R>(de, lnu, mu, &draws[slot].x0, kT, inv_kT);
             put(&r_sa[gh], (int32_t)sa);
             put(&r_sb[gh], (int32_t)na);
             put(&r_acc[gh], (int8_t)acc);
             put(&r_de[gh], de);
-            put(&r_ds[gh], (R)delta);  // the singlet change (one decoration)
+            put(&r_ds[gh], SFX ? (delta > 0 ? (R)2 : (R)-2) : (R)delta);  // the singlet change (one decoration)
           }
           acc = __shfl_sync(kFull, acc, LW * h);
           const uint32_t mark = (round << 6) | (uint32_t)(63 - gh);
@@ -1132,12 +1159,18 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
               }
               Dw[sp_e.eci] = delta * P;
             }
-            R sum = warp_sum(sp_coef * (R)P);
-            if (sd.singlet_eci >= 0) {
-              if (lane == 0) Dw[sd.singlet_eci] = SWAP ? 0 : delta;
-              if (!SWAP) sum += coef_s[sd.singlet_eci];
+            if (sd.singlet_eci >= 0 && lane == 0) Dw[sd.singlet_eci] = SWAP ? 0 : delta;
+            if (SFX && fx_scale != 0.0) {
+              long long sum = sp_cfx * (long long)P;
+#pragma unroll
+              for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
+              de_fx = (sum + sing_fx) * (long long)delta;
+              de = (R)((double)de_fx * fx_inv);
+            } else {
+              R sum = warp_sum(sp_coef * (R)P);
+              if (sd.singlet_eci >= 0 && !SWAP) sum += coef_s[sd.singlet_eci];
+              de = (R)delta * sum;
             }
-            de = (R)delta * sum;
           }
           int acc = 0;
           if (lane == 0) {
@@ -1148,7 +1181,7 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
             else
               acc = no_move ? 0
                             : (first ? 1
-                                     : (FX && fx_scale != 0.0 ? metropolis_fx(de_fx, de, ua, ub, kT, fx_kT)
+                                     : ((FX || SFX) && fx_scale != 0.0 ? metropolis_fx(de_fx, de, ua, ub, kT, fx_kT)
                                                               : metropolis<R>(de, ua, ub, kT, inv_kT)));
             if (CONS && no_move) put(&misc[3], 1);  // reported in the status at the end of the launch
             put(&r_sa[gidx], (int32_t)sa);
@@ -1158,7 +1191,7 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
             for (int b = 0; b < g.n_bf; ++b) {
               R v = (R)0;
               if constexpr (SPIN)
-                v = (R)(SWAP ? 0 : delta);
+                v = SWAP ? (R)0 : (delta > 0 ? (R)2 : (R)-2);
               else if constexpr (TAB)
                 v = SWAP ? (R)0 : bf_s[b * g.n_sym + na] - bf_s[b * g.n_sym + old_a];
               else if (g.singlet_eci[b] >= 0)

@@ -228,6 +228,21 @@ __global__ void __launch_bounds__(kSchedMaxThreads, 1) sched_kernel(DevGeo g, Ru
       ms[i] = m.z;
     }
     const R sing = sd.singlet_eci >= 0 ? coef_s[sd.singlet_eci] : (R)0;
+    constexpr bool FX = sizeof(R) == 8;  // FP64: energy changes in fixed point (fixed_point_scale)
+    double fx_inv = 0.0;                 // their quantum, 0: FP64 arithmetic
+    float fx_kT = 0.f;
+    long long coef_fx = 0, sing_fx = 0;
+    if constexpr (FX) {
+      // |P| is at most the ECI's terms, the spin change 2
+      const double most = warp_sum(lane < 8 ? 2.0 * fabs((double)coef) * (double)p_all : 0.0) + 2.0 * fabs((double)sing);
+      const double scale = fixed_point_scale(most, 0);
+      if (scale != 0.0) {
+        fx_inv = 1.0 / scale;
+        fx_kT = (float)(fx_inv / kT);
+        coef_fx = __double2ll_rn((double)coef * scale);
+        sing_fx = __double2ll_rn((double)sing * scale);
+      }
+    }
     const bool cols = 8 * hl < cp16;  // this lane's eight columns 8 hl .. 8 hl + 7 of a row
     const unsigned real = cols ? (1u << min(8, max(0, n_cols - 8 * hl))) - 1u : 0u;  // without the padding
     long long cf_acc = 0;
@@ -313,15 +328,27 @@ __global__ void __launch_bounds__(kSchedMaxThreads, 1) sched_kernel(DevGeo g, Ru
         }
         const int my_odd = is_multi ? (int)((odd64 >> fshift) & 255u) : 0;
         const int P = p_all - 2 * (__popc(wl & se.pair_lo) + __popc(wh & se.pair_hi) + my_odd);
-        R sum = coef * (R)P;
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
-        if (sd.singlet_eci >= 0) sum += sing;
         const int delta = ((uint32_t)oa ^ xorv) ? 2 : -2;
-        const R de = (R)delta * sum;
+        R de;
+        long long de_fx = 0;
+        if (FX && fx_inv != 0.0) {
+          long long sum = coef_fx * (long long)P;
+#pragma unroll
+          for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
+          de_fx = (sum + sing_fx) * (long long)delta;
+          de = (R)((double)de_fx * fx_inv);
+        } else {
+          R sum = coef * (R)P;
+#pragma unroll
+          for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
+          if (sd.singlet_eci >= 0) sum += sing;
+          de = (R)delta * sum;
+        }
         int acc = 0;
         if (hl == 0 && has) {
-          acc = metropolis_pre<R>(de, __uint_as_float(dr.y), __uint_as_float(dr.z), &uni[slot].x, kT, inv_kT);
+          const float lnu = __uint_as_float(dr.y), mu = __uint_as_float(dr.z);
+          acc = FX && fx_inv != 0.0 ? metropolis_pre_fx(de_fx, de, lnu, mu, &uni[slot].x, kT, fx_kT)
+                                    : metropolis_pre<R>(de, lnu, mu, &uni[slot].x, kT, inv_kT);
           const int na = oa ^ 1;
           if (acc) occ[sa] = (int8_t)na;
           r_acc[slot] = (uint8_t)(acc | (na << 1) | 4);

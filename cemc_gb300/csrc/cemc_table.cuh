@@ -73,17 +73,4 @@ __device__ __forceinline__ T table_sum(int S, const uint4 *geos, const T *F, con
   return sum;
 }
 
-// FP64 launches hold the table entries as int64 multiples of 2^-k: this part's FP64 pipe issues one warp
-// instruction in 16 cycles per SM, so 30 additions in each of 16 warps cost more than the rest of a round,
-// while 64-bit integer additions are two instructions on the wide pipe, and exact.  k is as large as sums
-// of 2 n entries of magnitude `most` allow (|sum| < 2^61), i.e. the quantum is at most 2^-60 n most: for 458
-// geometries of 0.1 eV 4e-17 eV, the spacing of FP64 numbers near 0.3 eV.  0: not representable (an ECI that
-// is infinite or NaN), the entries stay FP64.
-__device__ __forceinline__ double fixed_point_scale(double most, int n) {
-  const double bound = most * 2.0 * (double)(n + 1);
-  if (!(bound < 1e300)) return 0.0;
-  if (!(bound > 1e-200)) return 1.0;
-  return ldexp(1.0, 60 - ilogb(bound));
-}
-
 }  // namespace cemc
