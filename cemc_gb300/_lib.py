@@ -16,6 +16,7 @@ ERR_ARG = 1
 ERR_CUDA = 2
 ERR_BACKGROUND = 3
 ERR_STATE = 4
+CALC_CHANGES = 24  # changes one cemc_calculate or cemc_revert takes
 ERR_LIMIT = 5
 ERR_TIMEOUT = 6
 ERR_INTERNAL = 7
@@ -110,13 +111,17 @@ def load():
         L.cemc_energy.argtypes = [_P, C.c_int32, _P, _P, _P, _P]
         L.cemc_recompute_noalloc.argtypes = [_P, C.c_int32, _P, _P, _P, _P, _P]
         L.cemc_apply_changes.argtypes = [_P, _P, _P, _P, _P, C.c_int32, _P, _P, _P, _P, _P]
+        L.cemc_calculate.argtypes = [_P, _P, _P, _P, _P, C.c_int32, _P, _P, _P, _P, _P]
+        L.cemc_revert.argtypes = [_P, _P, _P, _P, _P, _P, C.c_int32, _P, _P, _P]
+        L.cemc_read.argtypes = [_P, _P, C.c_size_t, _P]
         L.cemc_delta_e.argtypes = [_P, _P, _P, C.c_int32, C.c_int32, C.c_int32, C.c_int32, _P, _P, _P]
         L.cemc_pt_exchange.argtypes = [C.c_int32, C.c_int32, C.c_uint64, C.c_uint64, _P, _P, _P, _P, _P, _P]
         L.cemc_last_error.argtypes = [C.c_char_p, C.c_size_t]
         L.cemc_version.argtypes = [C.POINTER(C.c_int32)] * 3
         for name in ("cemc_geometry_create", "cemc_geometry_destroy", "cemc_run", "cemc_recompute", "cemc_energy",
                      "cemc_recompute_noalloc",
-                     "cemc_apply_changes", "cemc_delta_e", "cemc_pt_exchange", "cemc_last_error", "cemc_version"):
+                     "cemc_apply_changes", "cemc_calculate", "cemc_revert", "cemc_read", "cemc_delta_e",
+                     "cemc_pt_exchange", "cemc_last_error", "cemc_version"):
             getattr(L, name).restype = C.c_int
         _lib = L
         return L
@@ -134,7 +139,8 @@ def exported_symbols():
     L = load()
     names = []
     for n in ("cemc_geometry_create", "cemc_geometry_destroy", "cemc_geometry_device_bytes", "cemc_run",
-              "cemc_recompute_scratch_doubles", "cemc_stamp_words", "cemc_recompute", "cemc_recompute_noalloc", "cemc_energy", "cemc_apply_changes", "cemc_delta_e", "cemc_pt_exchange", "cemc_last_error",
+              "cemc_recompute_scratch_doubles", "cemc_stamp_words", "cemc_recompute", "cemc_recompute_noalloc", "cemc_energy", "cemc_apply_changes",
+              "cemc_calculate", "cemc_revert", "cemc_read", "cemc_delta_e", "cemc_pt_exchange", "cemc_last_error",
               "cemc_version"):
         if hasattr(L, n):
             names.append(n)

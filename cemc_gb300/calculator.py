@@ -18,6 +18,7 @@ from __future__ import annotations
 
 import ctypes as C
 import json
+import threading
 from typing import Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -71,6 +72,12 @@ class DeviceUpdater:
         self.history: List[Tuple[int, int, int]] = []
         self._snap_cf = self.cf_d.clone()
         self._snap_energy = self.energy_d.clone()
+        # page-locked host memory the kernels and copies write results to: status and energy, then the
+        # correlation functions; one call uses it at a time
+        self._host = torch.zeros(2 + self.model.n_eci, dtype=torch.float64, pin_memory=True)
+        self._host_np = self._host.numpy()
+        self._host_lock = threading.Lock()
+        self._background = frozenset(int(i) for i in self.model.background)
 
     # -- device calls ----------------------------------------------------------
     def recompute(self):
@@ -83,28 +90,50 @@ class DeviceUpdater:
                                           _stream_ptr(self.stream)))
 
     def apply(self, changes: Sequence[Tuple[int, int, int]], record: bool = True):
-        """Apply (site, old id, new id) changes in order (``cemc_apply_changes``)."""
+        """Apply (site, old id, new id) changes in order.
+
+        Short lists (the moves of a Monte Carlo loop) go to the kernel as its arguments and the status
+        comes back through page-locked memory (``cemc_calculate``); longer ones through device arrays
+        (``cemc_apply_changes``).
+        """
         if not changes:
             return
-        arr = np.asarray(changes, dtype=np.int64).reshape(-1, 3)
-        if arr[:, 0].min() < 0 or arr[:, 0].max() >= self.model.n_sites:
+        self._apply(np.asarray(changes, dtype=np.int64).reshape(-1, 3).tolist(), record)
+
+    def _apply(self, rows, record=True) -> float:
+        """Apply a list of (site, old id, new id) and return the energy after them."""
+        n_sites = self.model.n_sites
+        if any(not 0 <= r[0] < n_sites for r in rows):
             raise IndexError("site index out of range")
-        if len(self.model.background) and np.isin(arr[:, 0], self.model.background).any():
+        if self._background and any(r[0] in self._background for r in rows):
             raise RuntimeError("Attempting to move a background atom!")
-        dev = self.occ_d.device
-        sites = torch.as_tensor(arr[:, 0].astype(np.int32)).to(dev)
-        old = torch.as_tensor(arr[:, 1].astype(np.int8)).to(dev)
-        new = torch.as_tensor(arr[:, 2].astype(np.int8)).to(dev)
-        _lib.check(self.geo.L.cemc_apply_changes(self.geo.handle, _ptr(self.occ_d), _ptr(self.cf_d),
-                                                 _ptr(self.energy_d), _ptr(self.eci_d), len(arr), _ptr(sites),
-                                                 _ptr(old), _ptr(new), _ptr(self.status_d), _stream_ptr(self.stream)))
-        st = int(self.status_d.item())
+        n, stream = len(rows), _stream_ptr(self.stream)
+        if n <= _lib.CALC_CHANGES:
+            sites, old, new = (C.c_int32 * n)(), (C.c_int8 * n)(), (C.c_int8 * n)()
+            for i, (s, o, w) in enumerate(rows):
+                sites[i], old[i], new[i] = s, o, w
+            with self._host_lock:
+                _lib.check(self.geo.L.cemc_calculate(self.geo.handle, _ptr(self.occ_d), _ptr(self.cf_d),
+                                                     _ptr(self.energy_d), _ptr(self.eci_d), n, sites, old, new,
+                                                     _ptr(self._host), stream))
+                st, energy = int(self._host_np[0]), float(self._host_np[1])
+        else:
+            arr = np.asarray(rows, dtype=np.int64)
+            dev = self.occ_d.device
+            sites = torch.as_tensor(arr[:, 0].astype(np.int32)).to(dev)
+            old = torch.as_tensor(arr[:, 1].astype(np.int8)).to(dev)
+            new = torch.as_tensor(arr[:, 2].astype(np.int8)).to(dev)
+            _lib.check(self.geo.L.cemc_apply_changes(self.geo.handle, _ptr(self.occ_d), _ptr(self.cf_d),
+                                                     _ptr(self.energy_d), _ptr(self.eci_d), n, _ptr(sites),
+                                                     _ptr(old), _ptr(new), _ptr(self.status_d), stream))
+            st, energy = int(self.status_d.item()), self.energy()
         if st == _lib.ERR_STATE:
             raise RuntimeError("The atom position tracker does not match the current state")
         if st:
             raise _lib.CemcError(st, "apply_changes failed")
         if record:
-            self.history.extend((int(s), int(o), int(n)) for s, o, n in arr)
+            self.history.extend((s, o, w) for s, o, w in rows)
+        return energy
 
     def delta_swap(self, a: int, b: int):
         _lib.check(self.geo.L.cemc_delta_e(self.geo.handle, _ptr(self.occ_d), _ptr(self.eci_d), _lib.MOVE_SWAP, a, b,
@@ -135,26 +164,37 @@ class DeviceUpdater:
     def undo(self) -> List[Tuple[int, int, int]]:
         """Revert every change since ``clear``; returns the reverted changes (latest first)."""
         undone = list(reversed(self.history))
-        if undone:
-            # each touched site returns to the species it had before its first change
-            first_old = {}
-            for s, o, _ in self.history:
-                first_old.setdefault(s, o)
+        # each touched site returns to the species it had before its first change
+        first_old = {}
+        for s, o, _ in self.history:
+            first_old.setdefault(s, o)
+        n = len(first_old)
+        if n > _lib.CALC_CHANGES:
             dev = self.occ_d.device
             sites = torch.as_tensor(np.fromiter(first_old.keys(), dtype=np.int64)).to(dev)
             olds = torch.as_tensor(np.fromiter(first_old.values(), dtype=np.int8)).to(dev)
             self.occ_d.index_copy_(0, sites, olds)
-        self.cf_d.copy_(self._snap_cf)
-        self.energy_d.copy_(self._snap_energy)
+            n = 0
+            first_old = {}
+        _lib.check(self.geo.L.cemc_revert(self.geo.handle, _ptr(self.occ_d), _ptr(self.cf_d), _ptr(self.energy_d),
+                                          _ptr(self._snap_cf), _ptr(self._snap_energy), n,
+                                          (C.c_int32 * n)(*first_old.keys()), (C.c_int8 * n)(*first_old.values()),
+                                          _stream_ptr(self.stream)))
         self.history.clear()
         return undone
 
     # -- host views --------------------------------------------------------------
+    def _read(self, src: torch.Tensor, at: int) -> np.ndarray:
+        n = src.numel()
+        with self._host_lock:
+            _lib.check(self.geo.L.cemc_read(self._host.data_ptr() + 8 * at, _ptr(src), n, _stream_ptr(self.stream)))
+            return self._host_np[at:at + n].copy()
+
     def cf(self) -> np.ndarray:
-        return self.cf_d.cpu().numpy()
+        return self._read(self.cf_d, 2)
 
     def energy(self) -> float:
-        return float(self.energy_d.item())
+        return float(self._read(self.energy_d, 1)[0])
 
     def occupation(self) -> np.ndarray:
         return self.occ_d.cpu().numpy()
@@ -237,9 +277,9 @@ class CE:
     def calculate(self, atoms=None, properties=None, system_changes=()):
         """Apply the changes and return the new energy (cemc/ce_calculator.py:345-364)."""
         changes = self._to_ids(system_changes)
-        self.updater.apply(changes)
+        energy = self.updater._apply(changes) if changes else self.updater.energy()
         self._mirror(changes)
-        self.results["energy"] = self.updater.energy()
+        self.results["energy"] = energy
         return self.results["energy"]
 
     def update_cf(self, single_change):

@@ -1400,8 +1400,62 @@ extern "C" int cemc_apply_changes(const cemc_geometry *geo, int8_t *occ, double 
     return fail(CEMC_ERR_ARG, "bad apply_changes arguments");
   if (cemc::warp_kernel_smem(geo->g) > (size_t)geo->max_smem) return fail(CEMC_ERR_LIMIT, "tables too large");
   cudaError_t e = cemc::launch_apply(geo->g, occ, cf, energy, eci, n_changes, sites, old_sym, new_sym, status,
-                                     static_cast<cudaStream_t>(stream));
+                                     (size_t)geo->max_smem, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "apply_changes kernel launch");
+  return CEMC_OK;
+}
+
+extern "C" int cemc_calculate(const cemc_geometry *geo, int8_t *occ, double *cf, double *energy, const double *eci,
+                              int32_t n_changes, const int32_t *sites, const int8_t *old_sym, const int8_t *new_sym,
+                              double *out, void *stream) {
+  if (!geo || !occ || !cf || !energy || !eci || !out || n_changes < 0 || n_changes > CEMC_CALC_CHANGES ||
+      (n_changes > 0 && (!sites || !old_sym || !new_sym)))
+    return fail(CEMC_ERR_ARG, "bad calculate arguments");
+  const cemc::DevGeo &g = geo->g;
+  if (cemc::warp_kernel_smem(g) > (size_t)geo->max_smem) return fail(CEMC_ERR_LIMIT, "tables too large");
+  cemc::ChangeArgs ch{};
+  ch.n = n_changes;
+  for (int i = 0; i < n_changes; ++i) {
+    if (sites[i] < 0 || sites[i] >= g.n_sites) return fail(CEMC_ERR_ARG, "site out of range");
+    if (new_sym[i] < 0 || new_sym[i] >= g.n_sym) return fail(CEMC_ERR_ARG, "bad species");
+    ch.site[i] = sites[i];
+    ch.old_sym[i] = old_sym[i];
+    ch.new_sym[i] = new_sym[i];
+  }
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  cudaError_t e = cemc::launch_calculate(g, occ, cf, energy, eci, ch, out, (size_t)geo->max_smem, st);
+  if (e != cudaSuccess) return cuda_fail(e, "calculate kernel launch");
+  e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) return cuda_fail(e, "calculate");
+  return CEMC_OK;
+}
+
+extern "C" int cemc_revert(const cemc_geometry *geo, int8_t *occ, double *cf, double *energy, const double *snap_cf,
+                           const double *snap_energy, int32_t n_sites, const int32_t *sites, const int8_t *sym,
+                           void *stream) {
+  if (!geo || !occ || !cf || !energy || !snap_cf || !snap_energy || n_sites < 0 || n_sites > CEMC_CALC_CHANGES ||
+      (n_sites > 0 && (!sites || !sym)))
+    return fail(CEMC_ERR_ARG, "bad revert arguments");
+  const cemc::DevGeo &g = geo->g;
+  cemc::ChangeArgs ch{};
+  ch.n = n_sites;
+  for (int i = 0; i < n_sites; ++i) {
+    if (sites[i] < 0 || sites[i] >= g.n_sites) return fail(CEMC_ERR_ARG, "site out of range");
+    ch.site[i] = sites[i];
+    ch.new_sym[i] = sym[i];
+  }
+  cudaError_t e = cemc::launch_revert(g.n_eci, occ, cf, energy, snap_cf, snap_energy, ch,
+                                      static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) return cuda_fail(e, "revert kernel launch");
+  return CEMC_OK;
+}
+
+extern "C" int cemc_read(double *dst, const double *src, size_t count, void *stream) {
+  if (count > 0 && (!dst || !src)) return fail(CEMC_ERR_ARG, "bad read arguments");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  cudaError_t e = cudaMemcpyAsync(dst, src, 8 * count, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) return cuda_fail(e, "read");
   return CEMC_OK;
 }
 

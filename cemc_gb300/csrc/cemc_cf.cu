@@ -250,43 +250,127 @@ __device__ WarpSmem warp_stage(const DevGeo &g, const double *eci, unsigned char
 }
 
 // Sequential single-site changes (CEUpdater::update_cf applied in order,
-// ce_updater.cpp:845-853), committed in place.  One warp.
-__global__ void apply_changes_kernel(DevGeo g, int8_t *occ, double *cf, double *energy, const double *eci,
-                                     int n_changes, const int32_t *sites, const int8_t *old_sym,
-                                     const int8_t *new_sym, int32_t *status) {
+// ce_updater.cpp:845-853), committed in place by one block.  The terms of a change are a serial chain
+// of dependent loads and FP64 products, so warp w of kApplyWarps walks the w-th part of every lane's chunk and the
+// parts of an ECI are added in a fixed order: two changes with 3,416 terms each took 63.9 us by one
+// warp and take 21.5, bound by the staging, the two gathers and the FP64 pipe.  The changes come
+// from device arrays or as kernel arguments.  Tables too large for the parts use one warp.
+constexpr int kApplyWarps = 8;
+
+int apply_warps(const DevGeo &g, size_t max_smem) {
+  const size_t more = 8 * (size_t)g.n_slots * 32 * kApplyWarps;
+  return warp_layout(g).total + more <= max_smem ? kApplyWarps : 1;
+}
+
+template <typename CHANGES>
+__device__ void apply_changes(const DevGeo &g, int8_t *occ, double *cf, double *energy, const double *eci,
+                              int n_changes, CHANGES change, int &rc, double &e_out) {
   extern __shared__ __align__(16) unsigned char smem[];
   WarpSmem s = warp_stage(g, eci, smem);
-  const int lane = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  double *part = s.part, *cf_s = s.d, *eci_s = s.coef;  // cf_s: the correlation functions while changes are applied
+  if (nw > 1) part = reinterpret_cast<double *>(smem + warp_layout(g).total);  // [nw][n_slots][32]
+  const int PS = g.n_slots * 32, LG = group_lane_ints(g.n_eci);
   int nbr[4];
-  int rc = 0;
+  rc = 0;
+  for (int k = tid; k < g.n_eci; k += blockDim.x) {
+    cf_s[k] = cf[k];
+    eci_s[k] = eci[k];
+  }
+  __syncthreads();
   for (int i = 0; i < n_changes; ++i) {
-    const int site = sites[i];
-    const int o = occ[site], n = new_sym[i];
-    if (o != old_sym[i]) {
+    int site, want, n;
+    change(i, site, want, n);
+    const int o = occ[site];
+    if (o != want) {
       rc = CEMC_ERR_STATE;
       break;
     }
     if (o == n) continue;
-    const int grp = g.n_groups > 1 ? g.site_group[site] : 0;
-    gather_vals<double>(g, occ, s.bf, site, o, n, -1, 0, s.va, nbr, lane);
-    __syncwarp();
-    site_changes<double, false>(g, s.terms, s.lane_term, s.kind, s.dec, s.coef, s.gscale, s.part, s.va, s.vb, s.d, grp,
-                                grp, lane);
-    for (int k = lane; k < g.n_eci; k += 32) {
-      const int kind = s.kind[k];
-      if (kind == 2) cf[k] = cf[k] + s.d[k] * g.eci_w[k];
-      else if (kind == 1) cf[k] = cf[k] + s.d[k] / (double)g.n_sites;
+    const int32_t *lt = s.lane_term + (g.n_groups > 1 ? g.site_group[site] : 0) * LG;
+    const double scale = s.gscale[g.n_groups > 1 ? g.site_group[site] : 0];
+    if (warp == 0) gather_vals<double>(g, occ, s.bf, site, o, n, -1, 0, s.va, nbr, lane);
+    __syncthreads();
+    {
+      double *my = part + warp * PS + lane;
+      for (int q = 0; q < g.n_slots; ++q) my[q * 32] = 0.0;
+      const int l0 = lt[lane], len = lt[lane + 1] - l0;
+      const int lo = l0 + len * warp / nw, hi = l0 + len * (warp + 1) / nw;
+      int cur = 0;
+      double acc = 0.0;
+      for (int t = lo; t < hi; ++t) {
+        const uint2 f = *reinterpret_cast<const uint2 *>(s.terms + 4 * t);
+        const int f0 = f.x & 0xffff, slot = f0 >> kRefBits;
+        if (slot != cur) {  // the terms of a lane are ordered by slot
+          my[cur * 32] = acc;
+          acc = 0.0;
+          cur = slot;
+        }
+        acc += s.va[f0 & ((1 << kRefBits) - 1)] * s.va[f.x >> 16] * s.va[f.y & 0xffff] * s.va[f.y >> 16];
+      }
+      my[cur * 32] = acc;
     }
-    __syncwarp();
-    if (lane == 0) occ[site] = (int8_t)n;
-    __syncwarp();
+    __syncthreads();
+    for (int k = tid; k < g.n_eci; k += blockDim.x) {
+      const int kind = s.kind[k];
+      if (kind == 2) {
+        double v = 0.0;
+        for (int l = lt[65 + 2 * k]; l <= lt[65 + 2 * k + 1]; ++l)
+          for (int w = 0; w < nw; ++w) v += part[w * PS + (k - lt[33 + l]) * 32 + l];
+        cf_s[k] += v * scale * g.eci_w[k];
+      } else if (kind == 1) {
+        cf_s[k] += s.va[g.one_idx + 1 + s.dec[k]] / (double)g.n_sites;
+      }
+    }
+    if (tid == 0) occ[site] = (int8_t)n;
+    __syncthreads();
   }
-  if (lane == 0) {
+  for (int k = tid; k < g.n_eci; k += blockDim.x) cf[k] = cf_s[k];
+  if (tid == 0) {
     double e = 0.0;
-    for (int k = 0; k < g.n_eci; ++k) e += eci[k] * cf[k];
-    *energy = e * (double)(unsigned)g.n_sites;
-    if (status) *status = rc;
+    for (int k = 0; k < g.n_eci; ++k) e += eci_s[k] * cf_s[k];
+    e_out = e * (double)(unsigned)g.n_sites;
+    *energy = e_out;
   }
+}
+
+__global__ void apply_changes_kernel(DevGeo g, int8_t *occ, double *cf, double *energy, const double *eci,
+                                     int n_changes, const int32_t *sites, const int8_t *old_sym,
+                                     const int8_t *new_sym, int32_t *status) {
+  int rc;
+  double e;
+  apply_changes(g, occ, cf, energy, eci, n_changes,
+                [&](int i, int &site, int &o, int &n) {
+                  site = sites[i];
+                  o = old_sym[i];
+                  n = new_sym[i];
+                },
+                rc, e);
+  if (threadIdx.x == 0 && status) *status = rc;
+}
+
+__global__ void calculate_kernel(DevGeo g, int8_t *occ, double *cf, double *energy, const double *eci, ChangeArgs ch,
+                                 double *out) {
+  int rc;
+  double e;
+  apply_changes(g, occ, cf, energy, eci, ch.n,
+                [&](int i, int &site, int &o, int &n) {
+                  site = ch.site[i];
+                  o = ch.old_sym[i];
+                  n = ch.new_sym[i];
+                },
+                rc, e);
+  if (threadIdx.x == 0) {
+    out[0] = (double)rc;
+    out[1] = e;
+  }
+}
+
+__global__ void revert_kernel(int n_eci, int8_t *occ, double *cf, double *energy, const double *snap_cf,
+                              const double *snap_energy, ChangeArgs ch) {
+  for (int k = threadIdx.x; k < n_eci; k += blockDim.x) cf[k] = snap_cf[k];
+  if ((int)threadIdx.x < ch.n) occ[ch.site[threadIdx.x]] = ch.new_sym[threadIdx.x];
+  if (threadIdx.x == 0) *energy = *snap_energy;
 }
 
 __global__ void delta_e_kernel(DevGeo g, const int8_t *occ, const double *eci, int move, int site_a, int site_b,
@@ -392,11 +476,28 @@ cudaError_t launch_recompute(const DevGeo &g, int n_chains, const int8_t *occ, c
 
 cudaError_t launch_apply(const DevGeo &g, int8_t *occ, double *cf, double *energy, const double *eci, int n,
                          const int32_t *sites, const int8_t *old_sym, const int8_t *new_sym, int32_t *status,
-                         cudaStream_t st) {
-  const size_t smem = warp_kernel_smem(g);
+                         size_t max_smem, cudaStream_t st) {
+  const int nw = apply_warps(g, max_smem);
+  const size_t smem = warp_kernel_smem(g) + (nw > 1 ? 8 * (size_t)g.n_slots * 32 * nw : 0);
   cudaError_t e = cudaFuncSetAttribute(apply_changes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  apply_changes_kernel<<<1, 32, smem, st>>>(g, occ, cf, energy, eci, n, sites, old_sym, new_sym, status);
+  apply_changes_kernel<<<1, 32 * nw, smem, st>>>(g, occ, cf, energy, eci, n, sites, old_sym, new_sym, status);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_calculate(const DevGeo &g, int8_t *occ, double *cf, double *energy, const double *eci,
+                             const ChangeArgs &ch, double *out, size_t max_smem, cudaStream_t st) {
+  const int nw = apply_warps(g, max_smem);
+  const size_t smem = warp_kernel_smem(g) + (nw > 1 ? 8 * (size_t)g.n_slots * 32 * nw : 0);
+  cudaError_t e = cudaFuncSetAttribute(calculate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  calculate_kernel<<<1, 32 * nw, smem, st>>>(g, occ, cf, energy, eci, ch, out);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_revert(int n_eci, int8_t *occ, double *cf, double *energy, const double *snap_cf,
+                          const double *snap_energy, const ChangeArgs &ch, cudaStream_t st) {
+  revert_kernel<<<1, 128, 0, st>>>(n_eci, occ, cf, energy, snap_cf, snap_energy, ch);
   return cudaGetLastError();
 }
 

@@ -279,6 +279,24 @@ int cemc_apply_changes(const cemc_geometry *geo, int8_t *occ, double *cf, double
                        int32_t n_changes, const int32_t *sites, const int8_t *old_sym, const int8_t *new_sym,
                        int32_t *status, void *stream);
 
+/* The same for at most CEMC_CALC_CHANGES changes given in host memory, and the result read back in the same
+ * call (CEUpdater::calculate returns the energy, ce_updater.cpp:471-519): the changes travel as kernel
+ * arguments, the kernel writes out[0] = CEMC_OK or CEMC_ERR_STATE and out[1] = energy to `out`, page-locked
+ * host memory the device can write, and the call returns when the stream has finished. */
+#define CEMC_CALC_CHANGES 24
+int cemc_calculate(const cemc_geometry *geo, int8_t *occ, double *cf, double *energy, const double *eci,
+                   int32_t n_changes, const int32_t *sites, const int8_t *old_sym, const int8_t *new_sym, double *out,
+                   void *stream);
+
+/* Take changes back (CFHistoryTracker, cf_history_tracker.cpp:46-149; CEUpdater::undo_changes,
+ * ce_updater.cpp:408-448): sites[i] (host memory, at most CEMC_CALC_CHANGES, each site once) returns to
+ * species sym[i], and cf and energy to the given device copies.  Asynchronous. */
+int cemc_revert(const cemc_geometry *geo, int8_t *occ, double *cf, double *energy, const double *snap_cf,
+                const double *snap_energy, int32_t n_sites, const int32_t *sites, const int8_t *sym, void *stream);
+
+/* Copy `count` doubles from device memory to page-locked host memory and wait for the stream. */
+int cemc_read(double *dst, const double *src, size_t count, void *stream);
+
 /* Energy change of a single flip or a swap without committing it (the
  * replay / debug path).  move: CEMC_MOVE_FLIP uses (site_a, new_a);
  * CEMC_MOVE_SWAP exchanges the species of site_a and site_b.  Writes the
