@@ -244,24 +244,22 @@ __device__ __forceinline__ int metropolis_fx(long long de_fx, R de, uint32_t ua,
 template <typename R>
 __device__ __forceinline__ int metropolis_pre(R de, float lnu, float mu, const uint32_t *uw, double kT,
                                               float inv_kT) {
-  if (de < (R)0) return 1;
   const float x = (float)de * inv_kT;
   const float y = lnu + x;
   const float margin = mu + 1e-6f * x;  // u == 0 gives an infinite margin
-  if (y < -margin) return 1;
-  if (y > margin) return 0;
+  const bool yes = de < (R)0 || y < -margin;
+  if (yes || y > margin) return yes;  // one branch, almost always taken
   return cemc_u01_53(uw[0], uw[1]) <= exp(-(double)de / kT);
 }
 // metropolis_pre() of an energy change held as an integer multiple of a quantum (see metropolis_fx).
 template <typename R>
 __device__ __forceinline__ int metropolis_pre_fx(long long de_fx, R de, float lnu, float mu, const uint32_t *uw,
                                                  double kT, float q_kT) {
-  if (de_fx < 0) return 1;
   const float x = (float)de_fx * q_kT;
   const float y = lnu + x;
   const float margin = mu + 1e-6f * x;  // u == 0 gives an infinite margin
-  if (y < -margin) return 1;
-  if (y > margin) return 0;
+  const bool yes = de_fx < 0 || y < -margin;
+  if (yes || y > margin) return yes;
   return cemc_u01_53(uw[0], uw[1]) <= exp(-(double)de / kT);
 }
 __device__ __forceinline__ void metropolis_parts(uint32_t ua, float &lnu, float &mu) {

@@ -48,8 +48,16 @@
 // each round (carrying the other half's totals), writes their trace entries,
 // and adds the correlation-function changes of its CTA's committed accepted
 // trials (change rows double-buffered by round parity) to a row of sums.
+// (In the spin form with one booker the fetcher adds the change rows.)
 // Correlation functions and energy are brought up to date in FP64 once, at
 // the end of the launch.
+//
+// A round of a small cell is one chain of dependent instructions per warp: 2,900 cycles for 4 to 8
+// trials of a 256- or 864-site cell, 535 warp instructions a trial, 1.2 issued per cycle and SM.  So the
+// two- and four-flip forms read the next trial's draw and row before the committed flips are stored,
+// select instead of branching, hold the multi-site terms in registers, and cells whose state is in shared memory have
+// their own build.  200 chains of 864 sites, 20 sweeps, FP32: 4.89 -> 3.97 ms; 100 chains of 2,048
+// sites by 16 warps, 5 sweeps: 2.40 -> 2.00 ms; one FP64 swap chain of 2,048 sites: 13.0 -> 12.2 ms.
 #include <cuda_runtime.h>
 
 #include <type_traits>
@@ -222,7 +230,10 @@ __device__ __forceinline__ double ld_peer_acc(const df64 *p, unsigned rank) {
 
 // CONS: this build runs the move-constraint redraw loop and the first-move acceptance (one
 // trial per warp, one CTA per chain); unconstrained launches take builds without them.
-template <typename R, int MOVE, int FORM, int CL, int TPW, bool CONS>
+// SH: the occupation, the conflict stamps and (swaps) the site lists are in shared memory, known at compile
+// time.  One build for both places reads them through generic pointers, whose 64-bit address arithmetic
+// was a tenth of a trial's instructions.
+template <typename R, int MOVE, int FORM, int CL, int TPW, bool CONS, bool SH>
 __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs a, SpinDev sd) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr bool SWAP = (MOVE == CEMC_MOVE_SWAP);
@@ -281,7 +292,7 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
   int32_t *rows = reinterpret_cast<int32_t *>(smem + L.rows);
   // two conflict-stamp tables of hmask + 1 entries: shared memory, or (large supercells,
   // exact) this chain's region of a global buffer shared by both CTAs of a pair
-  const bool gst = a.gstamp != nullptr;
+  const bool gst = !SH && a.gstamp != nullptr;
   uint32_t *stamp = gst ? a.gstamp + (size_t)chain * 2 * (hmask + 1) : reinterpret_cast<uint32_t *>(smem + L.stamp);
   unsigned char *rec0 = smem + L.rec;
   // change rows of this CTA's trials: exact integers in the spin basis
@@ -309,11 +320,11 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
   int32_t *sp_qtr_first = sp_qtr_term + 9;     // [8]
   const uint32_t xorv = SPIN ? (uint32_t)(sd.minus_id ^ 1) : 0u;  // spin bit = occ ^ xorv (1 = the -1 species)
 
-  int8_t *occ = a.occ_smem ? reinterpret_cast<int8_t *>(smem + L.occ) : a.occ + (size_t)chain * N;
+  int8_t *occ = SH || a.occ_smem ? reinterpret_cast<int8_t *>(smem + L.occ) : a.occ + (size_t)chain * N;
   int32_t *trk = nullptr, *loc = nullptr;
   if (SWAP) {
-    trk = a.trk_smem ? reinterpret_cast<int32_t *>(smem + L.trk) : a.trk + (size_t)chain * N;
-    loc = a.trk_smem ? trk + N : a.loc + (size_t)chain * N;
+    trk = SH || a.trk_smem ? reinterpret_cast<int32_t *>(smem + L.trk) : a.trk + (size_t)chain * N;
+    loc = SH || a.trk_smem ? trk + N : a.loc + (size_t)chain * N;
   }
 
   // A chain with no trials in this launch (an empty serving slot) leaves its
@@ -535,6 +546,7 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
     if (am) {
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
+        if (SPIN && o >= kh) break;  // lanes below kh take nothing from further lanes
         const R nx = __shfl_up_sync(kFull, x, o);
         R nd[NBF];
 #pragma unroll
@@ -682,6 +694,8 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
       }
     }
   };
+  // Spin form, one booker: the fetcher, which has the time, books the correlation functions.
+  const bool fetch_cf = SPIN && CL == 1 && NB == 1;
   auto book = [&](const unsigned char *rec, const DT *dbuf, int ks, uint64_t tb) {
     const int k0 = ks < 32 ? ks : 32, k1 = ks - k0;
     if (bq == 0) {
@@ -691,7 +705,8 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
       carry_half(rec, 0, k0);
       if (k1 > 0) book_half(rec, 32, k1, tb);
     }
-    if constexpr (!TAB) book_cf(rec, dbuf, ks);  // the table form leaves the CFs to a recompute
+    if constexpr (!TAB)
+      if (!fetch_cf) book_cf(rec, dbuf, ks);  // the table form leaves the CFs to a recompute
   };
 
   // Store into this CTA's shared memory and, in a pair, the peer's copy.
@@ -774,6 +789,35 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
     if constexpr (TPW <= 2 && !SWAP)
       sp_pk = __popc(sp_multi) <= 8 && __all_sync(kFull, el >= sd.n_cl || sp_e.n_multi <= 255);
   }
+  // Two or four flips per warp with at most four multi-site ECIs: the lane's terms in registers, each with
+  // its ECI's 8-bit field of one word, so that a count is a few dependent instructions: 330 cycles a round
+  // against 850 for the loop over the shared-memory copies, with counters of 6 bits and their repacking.
+  // More ECIs or terms (a lane of four-flip warps holds twice as many) take that loop: registers would spill.
+  constexpr int NTR = TPW == 2 ? 6 : (TPW == 4 ? 10 : 1);
+  bool sp_reg = false;
+  uint32_t tm_lo[NTR], tm_hi[NTR], tm_add[NTR], odd_mask = 0;
+  int odd_shift = 0;
+  R sing_c = (R)0;
+  if constexpr (TPW >= 2) {
+    const int el = lane % (32 / TPW);
+    sp_reg = __popc(sp_multi) <= 4 &&
+             __all_sync(kFull, (el >= sd.n_cl || sp_e.n_multi <= 255) && sp_thi - sp_tlo <= NTR);
+#pragma unroll
+    for (int i = 0; i < NTR; ++i) {
+      tm_lo[i] = tm_hi[i] = tm_add[i] = 0;
+      if (sp_tlo + i < sp_thi) {
+        const uint4 m = sp_terms[sp_tlo + i];
+        tm_lo[i] = m.x;
+        tm_hi[i] = m.y;
+        tm_add[i] = 1u << (8 * (__popc(sp_multi & ((1u << (sp_first + m.w / 6)) - 1u)) & 3));
+      }
+    }
+    if ((sp_multi >> el) & 1u) {
+      odd_mask = 255u;
+      odd_shift = 8 * (__popc(sp_multi & ((1u << el) - 1u)) & 3);
+    }
+    if (sd.singlet_eci >= 0) sing_c = coef_s[sd.singlet_eci];
+  }
   // Lane group of LW lanes: counters pa (and pb, the second site of a swap) of this lane's
   // terms, 6 bits per cluster ECI from sp_first on; the group's total for ECI el of each
   // multi-site ECI, in field (its rank among the multi-site ECIs) of one 64-bit word summed
@@ -805,6 +849,8 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
   // computes the same committed prefix `ks`, so the role loops below run in
   // lockstep.  Returns false when the launch is over, or when a pair's round
   // starts disagree (CEMC_ERR_INTERNAL, both CTAs stop at the same barrier).
+  int c_sa = 0, c_sb = 0;  // trial `lane` of the round: its site, new species (second site), flips: acceptance
+  bool c_acc = false;
   auto end_round = [&](uint32_t round, uint64_t t0, bool active, int &ks) -> bool {
     if (CL == 2) {
       if (tid == 0) st_peer(peer_addr(&t0_slot[round & 1], peer), t0);
@@ -820,19 +866,27 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
     const unsigned char *rec = rec0 + (size_t)(round & 1) * L.rec_stride;
     const int32_t *r_sa = reinterpret_cast<const int32_t *>(rec + L.rec_sa);
     const int32_t *r_sb = reinterpret_cast<const int32_t *>(rec + L.rec_sb);
+    const int8_t *r_acc = reinterpret_cast<const int8_t *>(rec + L.rec_acc);
     const uint32_t *tab = stamp + ((size_t)(round & 1) << L.stamp_bits);
     const int nv = (t_end - t0) < (uint64_t)CW ? (int)(t_end - t0) : CW;
-    auto conflicted = [&](int gg) {
-      const uint32_t v = tab[(uint32_t)r_sa[gg] & hmask];
+    auto conflicted = [&](int gg, int sa, int sb) {
+      const uint32_t v = tab[(uint32_t)sa & hmask];
       bool c = ((v >> 6) == round) && ((uint32_t)(63 - (v & 63u)) < (uint32_t)gg);
       if (SWAP) {
-        const uint32_t v2 = tab[(uint32_t)r_sb[gg] & hmask];
+        const uint32_t v2 = tab[(uint32_t)sb & hmask];
         c |= ((v2 >> 6) == round) && ((uint32_t)(63 - (v2 & 63u)) < (uint32_t)gg);
       }
       return c;
     };
-    const bool c0 = lane < nv && conflicted(lane);
-    const bool c1 = lane + 32 < nv && conflicted(lane + 32);
+    bool c0 = false;
+    c_acc = false;
+    if (lane < nv) {
+      c_sa = r_sa[lane];
+      c_sb = r_sb[lane];
+      if (!SWAP) c_acc = r_acc[lane] != 0;
+      c0 = conflicted(lane, c_sa, c_sb);
+    }
+    const bool c1 = lane + 32 < nv && conflicted(lane + 32, r_sa[lane + 32], SWAP ? r_sb[lane + 32] : 0);
     const unsigned m0 = __ballot_sync(kFull, c0);
     const unsigned m1 = __ballot_sync(kFull, c1);
     ks = m0 ? (__ffs(m0) - 1) : (m1 ? (31 + __ffs(m1)) : nv);
@@ -843,6 +897,29 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
   uint32_t round = 1;
   if (!helper) {
     // ---- evaluating warps: speculate, then apply the committed prefix ----------
+    // Two or four flips per warp: the draw and row of this lane group's next trial, read before the
+    // committed flips are stored (the compiler cannot move the reads past those stores)
+    constexpr int NJ = TPW >= 2 ? 2 * TPW : 1;  // column chunks of a neighbour row
+    uint4 n_dr = make_uint4(0u, 0u, 0u, 0u);
+    int n_nbr[NJ];
+    bool n_has = false;
+    auto load_trial = [&](uint64_t tr) {
+      if constexpr (TPW >= 2) {
+        constexpr int LW = 32 / TPW;
+        const uint64_t t = tr + (uint64_t)(rank * TPW * W + TPW * warp + lane / LW);
+        const uint32_t slot = (uint32_t)t & rmask;
+        n_has = t < t_end;
+        // slots past the last trial are read (they are in the ring) and not used: no branch
+        n_dr = *reinterpret_cast<const uint4 *>(&draws[slot]);  // site, w1, w2, w3
+        const int32_t *row = rows + slot * (uint32_t)cpad;
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+          const int c = lane % LW + LW * j, v = row[c < g.n_cols ? c : 0];
+          n_nbr[j] = n_has && c < g.n_cols ? v : -1;
+        }
+      }
+    };
+    load_trial(t0);
     while (true) {
       const bool active = t0 < t_end;
       unsigned char *rec = rec0 + (size_t)(round & 1) * L.rec_stride;
@@ -861,81 +938,78 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
       if constexpr (TPW >= 2) {
         // ---- phase A, TPW flips per warp: lane group h = lane / LW evaluates trial slot TPW warp + h ----
         constexpr int LW = 32 / TPW;      // lanes per trial (16 or 8)
-        constexpr int NJ = 64 / LW;       // column chunks of a neighbour row
         constexpr int FB = 32 / TPW;      // bits of a trial's field in the shared reductions
         constexpr uint32_t LMASK = (1u << LW) - 1u;
         if (active && t0 + (uint64_t)(rank * TPW * W + TPW * warp) < t_end) {
           const int h = lane / LW, hl = lane % LW;
           const int gh = rank * TPW * W + TPW * warp + h;  // trial slot in the round (pairs: CTA 1 after CTA 0)
-          const uint64_t t = t0 + (uint64_t)gh;
-          const bool has = t < t_end;  // the last groups of the last warp may have no trial
-          const uint32_t slot = (uint32_t)t & rmask;
-          int sa = 0, na = 0, oa = 0;
-          float lnu = 0.f, mu = 0.f;
-          if (has) {
-            const uint4 dr = *reinterpret_cast<const uint4 *>(&draws[slot]);  // site, w1, w2, w3
-            sa = (int)dr.x;
-            oa = occ[sa];
-            const int k = (int)cemc_below(dr.y, (uint32_t)(g.n_sym - 1));
-            na = k + (k >= oa);
-            lnu = __uint_as_float(dr.z);
-            mu = __uint_as_float(dr.w);
-          }
+          const bool has = n_has;  // the last groups of the last warp may have no trial
+          const uint32_t slot = (uint32_t)(t0 + (uint64_t)gh) & rmask;
+          const int sa = has ? (int)n_dr.x : 0, oa = occ[sa];
+          const int kk = (int)cemc_below(n_dr.y, (uint32_t)(g.n_sym - 1));
+          const int na = kk + (kk >= oa);
+          const float lnu = __uint_as_float(n_dr.z), mu = __uint_as_float(n_dr.w);
           const uint32_t occ_a_bit = (uint32_t)oa ^ xorv;
           // spin word of the neighbour row: bit c = column c, from NJ ballots of LW
           // columns (c = hl + LW j) of which each lane group keeps its own LW bits
-          const int32_t *row = rows + (size_t)slot * cpad;
           int nbr[NJ];
-          uint32_t wl = 0, wh = 0;
+          uint32_t wl = 0, wh = 0, bits[NJ];
 #pragma unroll
           for (int j = 0; j < NJ; ++j) {
-            const int c = hl + LW * j;
-            uint32_t bit = 0;
-            nbr[j] = -1;
-            if (has && c < g.n_cols) {
-              const int sn = row[c];
-              nbr[j] = sn;
-              bit = (uint32_t)occ[sn] ^ xorv;
-            }
-            const uint32_t chunk = (__ballot_sync(kFull, bit) >> (LW * h)) & LMASK;
+            nbr[j] = n_nbr[j];
+            const uint32_t o = (uint32_t)occ[nbr[j] >= 0 ? nbr[j] : 0] ^ xorv;
+            bits[j] = nbr[j] >= 0 ? o : 0u;
+          }
+#pragma unroll
+          for (int j = 0; j < NJ; ++j) {
+            const uint32_t chunk = (__ballot_sync(kFull, bits[j]) >> (LW * h)) & LMASK;
             if (LW * j < 32) wl |= chunk << (LW * j);
             else wh |= chunk << (LW * j - 32);
           }
-          const uint32_t pa = spin_lane_parities<true>(sp_terms, sp_tlo, sp_thi, wl, wh);
           // odd-parity counts of each multi-site cluster ECI: one reduction serves every
           // lane group (group h's count in bits FB h .. FB h + FB - 1; at most 255 when FB = 8)
           int my_odd = 0;
-          if constexpr (TPW == 4) {
-            // at most 8 cluster ECIs of at most 255 terms: every ECI's count in an 8-bit field
-            // of one 64-bit word, summed over the trial's 8 lanes by a butterfly (each partial
-            // sum is part of a total <= 255, so no field carries into the next)
-            uint64_t wsum = 0;
+          if (sp_reg) {
+            uint32_t wsum = 0;
 #pragma unroll
-            for (int sl = 0; sl < 5; ++sl)
-              if (sp_first + sl < 8) wsum |= (uint64_t)((pa >> (6 * sl)) & 63u) << (8 * (sp_first + sl));
-            if (sp_multi) {
+            for (int i = 0; i < NTR; ++i)
+              wsum += ((uint32_t)__popc((wl & tm_lo[i]) ^ (wh & tm_hi[i])) & 1u) * tm_add[i];
 #pragma unroll
-              for (int o = 1; o < LW; o <<= 1) wsum += __shfl_xor_sync(kFull, wsum, o);
-            }
-            my_odd = (int)((wsum >> (8 * (hl & 7))) & 255u);
-          } else if (sp_pk) {
-            my_odd = odd_counts_packed(pa, 0u, hl, std::integral_constant<int, LW>{});
+            for (int o = 1; o < LW; o <<= 1) wsum += __shfl_xor_sync(kFull, wsum, o);
+            my_odd = (int)((wsum >> odd_shift) & odd_mask);
           } else {
-            for (unsigned mm = sp_multi; mm; mm &= mm - 1) {
-              const int k = __ffs(mm) - 1;
-              const int sl = k - sp_first;
-              const uint32_t v = (sl >= 0 && sl < 5) ? ((pa >> (6 * sl)) & 63u) : 0u;
-              const uint32_t tot = __reduce_add_sync(kFull, v << (FB * h));
-              if (hl == k) my_odd = (int)((tot >> (FB * h)) & ((1u << FB) - 1u));
+            const uint32_t pa = spin_lane_parities<true>(sp_terms, sp_tlo, sp_thi, wl, wh);
+            if constexpr (TPW == 4) {
+              // at most 8 cluster ECIs of at most 255 terms: every ECI's count in an 8-bit field
+              // of one 64-bit word, summed over the trial's 8 lanes by a butterfly (each partial
+              // sum is part of a total <= 255, so no field carries into the next)
+              uint64_t wsum = 0;
+#pragma unroll
+              for (int sl = 0; sl < 5; ++sl)
+                if (sp_first + sl < 8) wsum |= (uint64_t)((pa >> (6 * sl)) & 63u) << (8 * (sp_first + sl));
+              if (sp_multi) {
+#pragma unroll
+                for (int o = 1; o < LW; o <<= 1) wsum += __shfl_xor_sync(kFull, wsum, o);
+              }
+              my_odd = (int)((wsum >> (8 * (hl & 7))) & 255u);
+            } else if (sp_pk) {
+              my_odd = odd_counts_packed(pa, 0u, hl, std::integral_constant<int, LW>{});
+            } else {
+              for (unsigned mm = sp_multi; mm; mm &= mm - 1) {
+                const int k = __ffs(mm) - 1;
+                const int sl = k - sp_first;
+                const uint32_t v = (sl >= 0 && sl < 5) ? ((pa >> (6 * sl)) & 63u) : 0u;
+                const uint32_t tot = __reduce_add_sync(kFull, v << (FB * h));
+                if (hl == k) my_odd = (int)((tot >> (FB * h)) & ((1u << FB) - 1u));
+              }
             }
           }
           const int delta = occ_a_bit ? 2 : -2;
           DT *Dh = dbuf + (size_t)(TPW * warp + h) * n_eci;  // this CTA's change row of the trial
-          int P = 0;
-          if (hl < sd.n_cl) {
-            P = sp_e.n_pairs - 2 * (__popc(wl & sp_e.pair_lo) + __popc(wh & sp_e.pair_hi)) + sp_e.n_multi - 2 * my_odd;
-            if (has) Dh[sp_e.eci] = delta * P;
-          }
+          // (0 on lanes without an ECI: their masks and counts are 0)
+          const int P = sp_e.n_pairs + sp_e.n_multi -
+                        2 * (__popc(wl & sp_e.pair_lo) + __popc(wh & sp_e.pair_hi) + (hl < sd.n_cl ? my_odd : 0));
+          if (hl < sd.n_cl && has) Dh[sp_e.eci] = delta * P;
           R de;
           long long de_fx = 0;
           if (SFX && fx_scale != 0.0) {
@@ -951,21 +1025,22 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
             for (int o = LW / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
             if (sd.singlet_eci >= 0) {
               if (hl == 0 && has) Dh[sd.singlet_eci] = delta;
-              sum += coef_s[sd.singlet_eci];
+              sum += sing_c;
             }
             de = (R)delta * sum;
           }
+          // every lane of the group has the trial's energy change and makes its test
           int acc = 0;
-          if (hl == 0 && has) {
+          if (has)
             acc = SFX && fx_scale != 0.0 ? metropolis_pre_fx(de_fx, de, lnu, mu, &draws[slot].x0, kT, fx_kT)
                                          : metropolis_pre<R>(de, lnu, mu, &draws[slot].x0, kT, inv_kT);
+          if (hl == 0 && has) {
             put(&r_sa[gh], (int32_t)sa);
             put(&r_sb[gh], (int32_t)na);
             put(&r_acc[gh], (int8_t)acc);
             put(&r_de[gh], de);
             put(&r_ds[gh], SFX ? (delta > 0 ? (R)2 : (R)-2) : (R)delta);  // the singlet change (one decoration)
           }
-          acc = __shfl_sync(kFull, acc, LW * h);
           const uint32_t mark = (round << 6) | (uint32_t)(63 - gh);
           if (CL == 1 && !gst) {
 #pragma unroll
@@ -1247,13 +1322,14 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
       if (!end_round(round, t0, active, ks)) break;
       // ---- phase B: apply every accepted move of the committed prefix ----------
       {
-        for (int gg = lane; gg < ks; gg += 32) {
-          if (r_acc[gg]) {
-            const int sa = r_sa[gg];
-            if (!SWAP) {
-              occ[sa] = (int8_t)r_sb[gg];
-            } else {
-              const int sb = r_sb[gg], A_ = r_A[gg], B_ = r_B[gg], la = r_la[gg], lb = r_lb[gg];
+        load_trial(t0 + (uint64_t)ks);
+        if constexpr (!SWAP) {
+          if (lane < ks && c_acc) occ[c_sa] = (int8_t)c_sb;
+          if (ks > 32 && lane + 32 < ks && r_acc[lane + 32]) occ[r_sa[lane + 32]] = (int8_t)r_sb[lane + 32];
+        } else {
+          for (int gg = lane; gg < ks; gg += 32) {
+            if (r_acc[gg]) {
+              const int sa = r_sa[gg], sb = r_sb[gg], A_ = r_A[gg], B_ = r_B[gg], la = r_la[gg], lb = r_lb[gg];
               occ[sa] = (int8_t)B_;
               occ[sb] = (int8_t)A_;
               trk[misc[12 + A_] + la] = sb;
@@ -1277,28 +1353,38 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
         book(rec0 + (size_t)((round - 1) & 1) * L.rec_stride, drow + (size_t)((round - 1) & 1) * TPW * W * n_eci,
              ks_prev, t0 - (uint64_t)ks_prev);
       if constexpr (SPIN)
-        if ((round & (kCfFoldRounds - 1)) == 0) cf_fold();
+        if (!fetch_cf && (round & (kCfFoldRounds - 1)) == 0) cf_fold();
       int ks;
       if (!end_round(round, t0, active, ks)) break;
       ks_prev = ks;
       t0 += (uint64_t)ks;
       ++round;
     }
+  } else {
+    // ---- fetcher: draws and neighbour rows kPrefetchRounds rounds ahead --------
+    int ks_prev = 0;
+    while (true) {
+      const bool active = t0 < t_end;
+      if (active) prefetch(t0);
+      if constexpr (SPIN) {
+        if (fetch_cf && round > 1)
+          book_cf(rec0 + (size_t)((round - 1) & 1) * L.rec_stride, drow + (size_t)((round - 1) & 1) * TPW * W * n_eci,
+                  ks_prev);
+        if (fetch_cf && (round & (kCfFoldRounds - 1)) == 0) cf_fold();
+      }
+      cp_async_wait_prev();
+      int ks;
+      if (!end_round(round, t0, active, ks)) break;
+      ks_prev = ks;
+      t0 += (uint64_t)ks;
+      ++round;
+    }
+  }
+  if (fetch_cf ? fetcher : booker) {
     if constexpr (SPIN) cf_fold();
     for (int i = 0; i < 4; ++i) {
       const int k = lane + 32 * i;
       if (k < n_eci) cfb[k] = cf_sum_out(cfr[i]);
-    }
-  } else {
-    // ---- fetcher: draws and neighbour rows kPrefetchRounds rounds ahead --------
-    while (true) {
-      const bool active = t0 < t_end;
-      if (active) prefetch(t0);
-      cp_async_wait_prev();
-      int ks;
-      if (!end_round(round, t0, active, ks)) break;
-      t0 += (uint64_t)ks;
-      ++round;
     }
   }
 
@@ -1389,7 +1475,10 @@ static unsigned block_threads(const RunArgs &a) {
 
 template <typename R, int MOVE, int FORM, int CL, int TPW, bool CONS = false>
 static cudaError_t launch_t(const DevGeo &g, const RunArgs &a, size_t smem, cudaStream_t st, const SpinDev &sd) {
-  auto k = mc_kernel<R, MOVE, FORM, CL, TPW, CONS>;
+  // the forms of ordinary runs have a build for cells whose state fits in shared memory
+  constexpr bool kBoth = (FORM == kFormSpin || FORM == kFormTable) && !CONS;
+  const bool sh = kBoth && a.occ_smem && !a.gstamp && (MOVE == CEMC_MOVE_FLIP || a.trk_smem);
+  auto k = sh ? mc_kernel<R, MOVE, FORM, CL, TPW, CONS, kBoth> : mc_kernel<R, MOVE, FORM, CL, TPW, CONS, false>;
   if (block_threads(a) > kMcMaxThreads) return cudaErrorInvalidConfiguration;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -1412,7 +1501,7 @@ static cudaError_t launch_t(const DevGeo &g, const RunArgs &a, size_t smem, cuda
 
 template <typename R, int MOVE, int FORM>
 static int clusters_t(const RunArgs &a, size_t smem) {
-  auto k = mc_kernel<R, MOVE, FORM, 2, 1, false>;
+  auto k = mc_kernel<R, MOVE, FORM, 2, 1, false, false>;  // (the same threads, registers bound and memory as its other build)
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(a.n_chains * 2));
@@ -1466,20 +1555,11 @@ static cudaError_t launch_recycle(const DevGeo &g, const RunArgs &a, int move, s
                                 : launch_t<R, CEMC_MOVE_FLIP, kFormRecycle, 1, 1, true>(g, a, smem, st, none);
 }
 
-cudaError_t launch_mc(const DevGeo &g, const RunArgs &a, int move, int precision, size_t smem, cudaStream_t st,
-                      int form, const SpinDev *spin) {
-  // two trials per warp: spin flips on one CTA per chain only (checked by the caller)
-  if (a.tpw >= 2 && (form != kFormSpin || move != CEMC_MOVE_FLIP || a.cons)) return cudaErrorInvalidValue;
-  if (a.tpw == 4 && a.cl != 1) return cudaErrorInvalidValue;
-  if (a.cons && a.cl != 1) return cudaErrorInvalidValue;
-  if (form == kFormSpin && !spin) return cudaErrorInvalidValue;
-  if (form == kFormRecycle) {
-    if (a.cl != 1 || a.tpw != 1) return cudaErrorInvalidValue;
-    return precision == CEMC_PREC_F32 ? launch_recycle<float>(g, a, move, smem, st)
-                                      : launch_recycle<double>(g, a, move, smem, st);
-  }
-  return precision == CEMC_PREC_F32 ? launch_r<float>(g, a, move, smem, st, form, spin)
-                                    : launch_r<double>(g, a, move, smem, st, form, spin);
+// One precision: the two are compiled as two units, at the same time (CEMC_MC_F64 for the FP64 one).
+template <typename R>
+cudaError_t launch_precision(const DevGeo &g, const RunArgs &a, int move, size_t smem, cudaStream_t st, int form,
+                             const SpinDev *spin) {
+  return form == kFormRecycle ? launch_recycle<R>(g, a, move, smem, st) : launch_r<R>(g, a, move, smem, st, form, spin);
 }
 
 template <typename R, int FORM>
@@ -1487,11 +1567,38 @@ static int clusters_m(const RunArgs &a, int move, size_t smem) {
   return move == CEMC_MOVE_SWAP ? clusters_t<R, CEMC_MOVE_SWAP, FORM>(a, smem) : clusters_t<R, CEMC_MOVE_FLIP, FORM>(a, smem);
 }
 
-int max_active_clusters(const DevGeo &, const RunArgs &a, int move, int precision, size_t smem, int form) {
-  const bool f32 = precision == CEMC_PREC_F32;
-  if (form == kFormSpin) return f32 ? clusters_m<float, kFormSpin>(a, move, smem) : clusters_m<double, kFormSpin>(a, move, smem);
-  if (form == kFormTable) return f32 ? clusters_m<float, kFormTable>(a, move, smem) : clusters_m<double, kFormTable>(a, move, smem);
-  return f32 ? clusters_m<float, kFormGeneric>(a, move, smem) : clusters_m<double, kFormGeneric>(a, move, smem);
+template <typename R>
+int clusters_precision(const RunArgs &a, int move, size_t smem, int form) {
+  if (form == kFormSpin) return clusters_m<R, kFormSpin>(a, move, smem);
+  if (form == kFormTable) return clusters_m<R, kFormTable>(a, move, smem);
+  return clusters_m<R, kFormGeneric>(a, move, smem);
 }
+
+#ifdef CEMC_MC_F64
+template cudaError_t launch_precision<double>(const DevGeo &, const RunArgs &, int, size_t, cudaStream_t, int,
+                                              const SpinDev *);
+template int clusters_precision<double>(const RunArgs &, int, size_t, int);
+#else
+extern template cudaError_t launch_precision<double>(const DevGeo &, const RunArgs &, int, size_t, cudaStream_t, int,
+                                                     const SpinDev *);
+extern template int clusters_precision<double>(const RunArgs &, int, size_t, int);
+
+cudaError_t launch_mc(const DevGeo &g, const RunArgs &a, int move, int precision, size_t smem, cudaStream_t st,
+                      int form, const SpinDev *spin) {
+  // two trials per warp: spin flips on one CTA per chain only (checked by the caller)
+  if (a.tpw >= 2 && (form != kFormSpin || move != CEMC_MOVE_FLIP || a.cons)) return cudaErrorInvalidValue;
+  if (a.tpw == 4 && a.cl != 1) return cudaErrorInvalidValue;
+  if (a.cons && a.cl != 1) return cudaErrorInvalidValue;
+  if (form == kFormSpin && !spin) return cudaErrorInvalidValue;
+  if (form == kFormRecycle && (a.cl != 1 || a.tpw != 1)) return cudaErrorInvalidValue;
+  return precision == CEMC_PREC_F32 ? launch_precision<float>(g, a, move, smem, st, form, spin)
+                                    : launch_precision<double>(g, a, move, smem, st, form, spin);
+}
+
+int max_active_clusters(const DevGeo &, const RunArgs &a, int move, int precision, size_t smem, int form) {
+  return precision == CEMC_PREC_F32 ? clusters_precision<float>(a, move, smem, form)
+                                    : clusters_precision<double>(a, move, smem, form);
+}
+#endif
 
 }  // namespace cemc
