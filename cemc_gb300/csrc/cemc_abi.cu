@@ -169,8 +169,9 @@ extern "C" int cemc_geometry_create(const cemc_geometry_desc *d, cemc_geometry *
     std::vector<int> lo_seen(K, 33), hi_seen(K, -1);
     for (int l = 0; l < 32; ++l) {
       const int lo = lt[l], hi = lt[l + 1];
+      // a lane without terms (fewer than 32) between two lanes of an ECI is read as that ECI's slot 0
+      if (lo < t0 + Tg) fi[l] = d->term_eci[lo];
       if (lo >= hi) continue;
-      fi[l] = d->term_eci[lo];
       n_slots = std::max(n_slots, d->term_eci[hi - 1] - fi[l] + 1);
       for (int i = lo; i < hi; ++i) {
         const int k = d->term_eci[i];

@@ -18,6 +18,8 @@ def _updater(system):
     from cemc_gb300.tables import CEModel
     if system == "hcp":
         s = hcp_settings(6, 5, 2, 1, 1, ["Al", "Mg", "Si"])
+    elif system == "pairs":  # 12 terms: lanes without any between the lanes of one ECI
+        s = fcc_settings(4, 1, 0, 0, ["Al", "Mg"])
     elif system == "ternary":
         s = fcc_settings(5, 5, 3, 1, ["Al", "Mg", "Si"])
     else:
@@ -29,7 +31,7 @@ def _updater(system):
     return DeviceUpdater(E.Geometry(m, "cuda"), occ, m.eci_vector(eci)), m, m.eci_vector(eci), occ, rng
 
 
-@pytest.mark.parametrize("system", ["binary", "ternary", "hcp"])
+@pytest.mark.parametrize("system", ["binary", "pairs", "ternary", "hcp"])
 @pytest.mark.parametrize("n", [1, 2, 24, 25])
 def test_changes_and_undo(system, n):
     from cemc_gb300.calculator import DeviceUpdater
