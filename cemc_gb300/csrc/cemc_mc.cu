@@ -57,7 +57,9 @@
 // two- and four-flip forms read the next trial's draw and row before the committed flips are stored,
 // select instead of branching, hold the multi-site terms in registers, and cells whose state is in shared memory have
 // their own build.  200 chains of 864 sites, 20 sweeps, FP32: 4.89 -> 3.97 ms; 100 chains of 2,048
-// sites by 16 warps, 5 sweeps: 2.40 -> 2.00 ms; one FP64 swap chain of 2,048 sites: 13.0 -> 12.2 ms.
+// sites by 16 warps, 5 sweeps: 2.40 -> 2.00 ms.  Swaps: the fetcher turns a draw into species, list slots
+// and the acceptance test's parts, and one reduction gives the two sites' differences of counts: one
+// FP64 chain of 2,048 sites, 10 sweeps, 13.0 -> 10.1 ms.
 #include <cuda_runtime.h>
 
 #include <type_traits>
@@ -474,21 +476,29 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
         d.x0 = w1.v[0];
         d.x1 = w1.v[1];
         d.site = -1;
-        // The sites are read from the site lists when the trial is evaluated, rounds from
-        // now; the lists' extents do not change (swaps keep every species count), so the
-        // sites at the trial's two list slots now are almost always the ones it will
-        // read: warm L1 with their neighbour rows.  Only a hint; a stale guess costs the
-        // L2 latency the evaluation pays without it.
-        const int np = misc[2];
-        if (np >= 2) {
-          const int ia = (int)cemc_below(w0.v[0], (uint32_t)np);
-          int ib = (int)cemc_below(w0.v[1], (uint32_t)(np - 1));
-          ib += (ib >= ia);
-          const int A = misc[4 + ia], B = misc[4 + ib];
-          const int pa = trk[misc[12 + A] + (int)cemc_below(w0.v[2], (uint32_t)misc[20 + A])];
-          const int pb = trk[misc[12 + B] + (int)cemc_below(w0.v[3], (uint32_t)misc[20 + B])];
-          if (g.box_L == 0 && (unsigned)pa < (unsigned)N) prefetch_row(g.table + (size_t)pa * cpad, cpad);
-          if (g.box_L == 0 && (unsigned)pb < (unsigned)N) prefetch_row(g.table + (size_t)pb * cpad, cpad);
+        // The two species and list slots: the lists' extents do not change (swaps keep every
+        // species count), so only the sites in the slots are left to the evaluation.
+        const int np = misc[2];  // at least two (checked before the first trial)
+        const int ia = (int)cemc_below(w0.v[0], (uint32_t)np);
+        int ib = (int)cemc_below(w0.v[1], (uint32_t)(np - 1));
+        ib += (ib >= ia);
+        const int A = misc[4 + ia], B = misc[4 + ib];
+        d.w0 = (uint32_t)A | ((uint32_t)B << 8);
+        d.w2 = (uint32_t)misc[12 + A] + cemc_below(w0.v[2], (uint32_t)misc[20 + A]);
+        d.w3 = (uint32_t)misc[12 + B] + cemc_below(w0.v[3], (uint32_t)misc[20 + B]);
+        if constexpr (!CONS) {  // the acceptance test's parts of the uniform
+          float lnu, mu;
+          metropolis_parts(d.x0, lnu, mu);
+          d.site = (int)__float_as_uint(lnu);
+          d.pad = __float_as_uint(mu);
+        }
+        // The sites in the slots now are almost always the ones the trial will read: warm L1 with
+        // their neighbour rows.  Only a hint; a stale guess costs the L2 latency the evaluation
+        // pays without it.
+        if (g.box_L == 0) {
+          const int pa = trk[d.w2], pb = trk[d.w3];
+          if ((unsigned)pa < (unsigned)N) prefetch_row(g.table + (size_t)pa * cpad, cpad);
+          if ((unsigned)pb < (unsigned)N) prefetch_row(g.table + (size_t)pb * cpad, cpad);
         }
       } else {
         d.x0 = d.x1 = 0;
@@ -789,19 +799,19 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
     if constexpr (TPW <= 2 && !SWAP)
       sp_pk = __popc(sp_multi) <= 8 && __all_sync(kFull, el >= sd.n_cl || sp_e.n_multi <= 255);
   }
-  // Two or four flips per warp with at most four multi-site ECIs: the lane's terms in registers, each with
+  // At most four multi-site ECIs and NTR terms a lane: the lane's terms in registers, each with
   // its ECI's 8-bit field of one word, so that a count is a few dependent instructions: 330 cycles a round
   // against 850 for the loop over the shared-memory copies, with counters of 6 bits and their repacking.
   // More ECIs or terms (a lane of four-flip warps holds twice as many) take that loop: registers would spill.
-  constexpr int NTR = TPW == 2 ? 6 : (TPW == 4 ? 10 : 1);
+  constexpr int NTR = TPW == 2 ? 6 : (TPW == 4 ? 10 : 4);
   bool sp_reg = false;
   uint32_t tm_lo[NTR], tm_hi[NTR], tm_add[NTR], odd_mask = 0;
   int odd_shift = 0;
   R sing_c = (R)0;
-  if constexpr (TPW >= 2) {
+  if constexpr (SPIN) {
     const int el = lane % (32 / TPW);
     sp_reg = __popc(sp_multi) <= 4 &&
-             __all_sync(kFull, (el >= sd.n_cl || sp_e.n_multi <= 255) && sp_thi - sp_tlo <= NTR);
+             __all_sync(kFull, (el >= sd.n_cl || sp_e.n_multi <= (SWAP ? 127 : 255)) && sp_thi - sp_tlo <= NTR);
 #pragma unroll
     for (int i = 0; i < NTR; ++i) {
       tm_lo[i] = tm_hi[i] = tm_add[i] = 0;
@@ -809,7 +819,7 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
         const uint4 m = sp_terms[sp_tlo + i];
         tm_lo[i] = m.x;
         tm_hi[i] = m.y;
-        tm_add[i] = 1u << (8 * (__popc(sp_multi & ((1u << (sp_first + m.w / 6)) - 1u)) & 3));
+        tm_add[i] = 1u << (8 * (__popc(sp_multi & ((1u << (sp_first + (TPW == 1 ? m.z : m.w) / 6)) - 1u)) & 3));
       }
     }
     if ((sp_multi >> el) & 1u) {
@@ -1110,13 +1120,10 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
               spin_ballot(g, occ, row_mem(frow), xorv, -1, 0u, wa_lo, wa_hi, nbra, lane);
             }
           } else {
-            int ia = (int)cemc_below(dr.w0, (uint32_t)n_present);
-            int ib = (int)cemc_below(dr.w1, (uint32_t)(n_present - 1));
-            ib += (ib >= ia);
-            A_ = misc[4 + ia];
-            B_ = misc[4 + ib];
-            sa = trk[misc[12 + A_] + (int)cemc_below(dr.w2, (uint32_t)misc[20 + A_])];
-            sb = trk[misc[12 + B_] + (int)cemc_below(dr.w3, (uint32_t)misc[20 + B_])];
+            A_ = (int)(dr.w0 & 255u);
+            B_ = (int)(dr.w0 >> 8);
+            sa = trk[dr.w2];
+            sb = trk[dr.w3];
             ua = dr.x0;
             ub = dr.x1;
             if (cons) {
@@ -1126,8 +1133,8 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
                 ++att;
                 const cemc_u32x4 w = cemc_trial_draw(a.seed, key, t, (uint32_t)(2 * att));
                 const cemc_u32x4 x = cemc_trial_draw(a.seed, key, t, (uint32_t)(2 * att + 1));
-                ia = (int)cemc_below(w.v[0], (uint32_t)n_present);
-                ib = (int)cemc_below(w.v[1], (uint32_t)(n_present - 1));
+                const int ia = (int)cemc_below(w.v[0], (uint32_t)n_present);
+                int ib = (int)cemc_below(w.v[1], (uint32_t)(n_present - 1));
                 ib += (ib >= ia);
                 A_ = misc[4 + ia];
                 B_ = misc[4 + ib];
@@ -1207,13 +1214,23 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
             // masks, its multi-site terms from one warp reduction per ECI that has any.
             delta = ((occ_a_bit) ? 2 : -2);
             const int first = sp_first;
-            const uint32_t pa = spin_lane_parities<false>(sp_terms, sp_tlo, sp_thi, wa_lo, wa_hi);
-            const uint32_t pb = SWAP ? spin_lane_parities<false>(sp_terms, sp_tlo, sp_thi, wb_lo, wb_hi) : 0u;
             int my_odd = 0;
-            if (sp_pk) {
-              my_odd = odd_counts_packed(pa, pb, lane, std::integral_constant<int, 32>{});
+            if (sp_reg) {
+              // swaps: differences of the two sites' counts, biased by 128 so that no field borrows
+              uint32_t wsum = 0;
+#pragma unroll
+              for (int i = 0; i < NTR; ++i) {
+                int d = __popc((wa_lo & tm_lo[i]) ^ (wa_hi & tm_hi[i])) & 1;
+                if (SWAP) d -= __popc((wb_lo & tm_lo[i]) ^ (wb_hi & tm_hi[i])) & 1;
+                wsum += (uint32_t)d * tm_add[i];
+              }
+              const uint32_t tot = __reduce_add_sync(kFull, wsum) + (SWAP ? 0x80808080u : 0u);
+              my_odd = (int)((tot >> odd_shift) & odd_mask) - (SWAP ? (int)(odd_mask & 128u) : 0);
             } else {
-              for (unsigned mm = sp_multi; mm; mm &= mm - 1) {
+              const uint32_t pa = spin_lane_parities<false>(sp_terms, sp_tlo, sp_thi, wa_lo, wa_hi);
+              const uint32_t pb = SWAP ? spin_lane_parities<false>(sp_terms, sp_tlo, sp_thi, wb_lo, wb_hi) : 0u;
+              if (sp_pk) my_odd = odd_counts_packed(pa, pb, lane, std::integral_constant<int, 32>{});
+              for (unsigned mm = sp_pk ? 0u : sp_multi; mm; mm &= mm - 1) {
                 const int k = __ffs(mm) - 1;
                 const int sl = k - first;
                 int v = (sl >= 0 && sl < 5) ? (int)((pa >> (6 * sl)) & 63u) : 0;
@@ -1251,13 +1268,18 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
           if (lane == 0) {
             // accept_first_trial_move_after_reset: the call's first trial is accepted outright
             const bool first = CONS && a.accept_first && a.chunk_offset == 0 && t == t_first;
-            if constexpr (RECYCLE)
+            if constexpr (RECYCLE) {
               acc = no_move ? 0 : (first ? 1 : barker<R>(de, ua, ub, kT));
-            else
+            } else if constexpr (SWAP && !CONS) {
+              const float lnu = __uint_as_float((uint32_t)dr.site), mu = __uint_as_float(dr.pad);
+              acc = (FX || SFX) && fx_scale != 0.0 ? metropolis_pre_fx(de_fx, de, lnu, mu, &draws[slot].x0, kT, fx_kT)
+                                                   : metropolis_pre<R>(de, lnu, mu, &draws[slot].x0, kT, inv_kT);
+            } else {
               acc = no_move ? 0
                             : (first ? 1
                                      : ((FX || SFX) && fx_scale != 0.0 ? metropolis_fx(de_fx, de, ua, ub, kT, fx_kT)
                                                               : metropolis<R>(de, ua, ub, kT, inv_kT)));
+            }
             if (CONS && no_move) put(&misc[3], 1);  // reported in the status at the end of the launch
             put(&r_sa[gidx], (int32_t)sa);
             put(&r_sb[gidx], (int32_t)(SWAP ? sb : na));
