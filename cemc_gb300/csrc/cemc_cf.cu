@@ -474,12 +474,13 @@ cudaError_t launch_recompute(const DevGeo &g, int n_chains, const int8_t *occ, c
   return cudaGetLastError();
 }
 
+// (The bound is the device's, not the launch's: threads with other geometries set the same value.)
 cudaError_t launch_apply(const DevGeo &g, int8_t *occ, double *cf, double *energy, const double *eci, int n,
                          const int32_t *sites, const int8_t *old_sym, const int8_t *new_sym, int32_t *status,
                          size_t max_smem, cudaStream_t st) {
   const int nw = apply_warps(g, max_smem);
   const size_t smem = warp_kernel_smem(g) + (nw > 1 ? 8 * (size_t)g.n_slots * 32 * nw : 0);
-  cudaError_t e = cudaFuncSetAttribute(apply_changes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(apply_changes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
   if (e != cudaSuccess) return e;
   apply_changes_kernel<<<1, 32 * nw, smem, st>>>(g, occ, cf, energy, eci, n, sites, old_sym, new_sym, status);
   return cudaGetLastError();
@@ -489,7 +490,7 @@ cudaError_t launch_calculate(const DevGeo &g, int8_t *occ, double *cf, double *e
                              const ChangeArgs &ch, double *out, size_t max_smem, cudaStream_t st) {
   const int nw = apply_warps(g, max_smem);
   const size_t smem = warp_kernel_smem(g) + (nw > 1 ? 8 * (size_t)g.n_slots * 32 * nw : 0);
-  cudaError_t e = cudaFuncSetAttribute(calculate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(calculate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
   if (e != cudaSuccess) return e;
   calculate_kernel<<<1, 32 * nw, smem, st>>>(g, occ, cf, energy, eci, ch, out);
   return cudaGetLastError();
