@@ -1325,28 +1325,28 @@ extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream
     tick_smem = cemc::tick_layout(g, is_swap, rsize, tick.row_bits, tick.head_bits).total;
   for (uint64_t done = 0; done < r->n_trials;) {
     const uint64_t n = std::min(max_chunk, r->n_trials - done);
+    cudaError_t e;
     if (tick_smem) {
       tick.n_trials = n;
       tick.chunk_offset = done;
-      cudaError_t e = cemc::launch_tick(g, tick, r->move, r->precision, tick_smem, static_cast<cudaStream_t>(stream));
+      e = cemc::launch_tick(g, tick, r->move, r->precision, tick_smem, static_cast<cudaStream_t>(stream));
       if (e != cudaSuccess) return cuda_fail(e, "scheduled table kernel launch");
-      done += n;
-      continue;
+    } else {
+      a.n_trials = n;
+      a.chunk_offset = done;
+      e = cemc::launch_mc(g, a, r->move, r->precision, L.total, static_cast<cudaStream_t>(stream), form,
+                          use_spin ? &geo->spin : nullptr);
+      if (e != cudaSuccess) return cuda_fail(e, "Monte Carlo kernel launch");
     }
-    a.n_trials = n;
-    a.chunk_offset = done;
-    cudaError_t e = cemc::launch_mc(g, a, r->move, r->precision, L.total, static_cast<cudaStream_t>(stream), form,
-                                    use_spin ? &geo->spin : nullptr);
-    if (e != cudaSuccess) return cuda_fail(e, "Monte Carlo kernel launch");
     done += n;
+    if (form == cemc::kFormTable) {  // after every launch: the next one's sums start from cf and energy
+      e = recompute(geo, r->n_chains, r->occ, r->eci, r->cf, r->energy, rscratch, stream);
+      if (e != cudaSuccess) return cuda_fail(e, "recompute after the table kernel");
+    }
   }
   r->kernel_used = form == cemc::kFormTable ? CEMC_KERNEL_TABLE
                   : (form == cemc::kFormGeneric || form == cemc::kFormRecycle) ? CEMC_KERNEL_GENERIC
                   : (a.tpw == 4 ? CEMC_KERNEL_SPIN_QUARTER : a.tpw == 2 ? CEMC_KERNEL_SPIN_HALFWARP : CEMC_KERNEL_SPIN);
-  if (form == cemc::kFormTable) {
-    cudaError_t e = recompute(geo, r->n_chains, r->occ, r->eci, r->cf, r->energy, rscratch, stream);
-    if (e != cudaSuccess) return cuda_fail(e, "recompute after the table kernel");
-  }
   return CEMC_OK;
 }
 
