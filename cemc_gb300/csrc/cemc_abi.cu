@@ -918,6 +918,7 @@ extern "C" int cemc_geometry_create(const cemc_geometry_desc *d, cemc_geometry *
   int dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&geo->max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  geo->g.max_smem = geo->max_smem;
   cudaDeviceGetAttribute(&geo->n_sms, cudaDevAttrMultiProcessorCount, dev);
   *out = geo;
   return CEMC_OK;
@@ -1401,7 +1402,7 @@ extern "C" int cemc_apply_changes(const cemc_geometry *geo, int8_t *occ, double 
     return fail(CEMC_ERR_ARG, "bad apply_changes arguments");
   if (cemc::warp_kernel_smem(geo->g) > (size_t)geo->max_smem) return fail(CEMC_ERR_LIMIT, "tables too large");
   cudaError_t e = cemc::launch_apply(geo->g, occ, cf, energy, eci, n_changes, sites, old_sym, new_sym, status,
-                                     (size_t)geo->max_smem, static_cast<cudaStream_t>(stream));
+                                     static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "apply_changes kernel launch");
   return CEMC_OK;
 }
@@ -1424,7 +1425,7 @@ extern "C" int cemc_calculate(const cemc_geometry *geo, int8_t *occ, double *cf,
     ch.new_sym[i] = new_sym[i];
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  cudaError_t e = cemc::launch_calculate(g, occ, cf, energy, eci, ch, out, (size_t)geo->max_smem, st);
+  cudaError_t e = cemc::launch_calculate(g, occ, cf, energy, eci, ch, out, st);
   if (e != cudaSuccess) return cuda_fail(e, "calculate kernel launch");
   e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return cuda_fail(e, "calculate");

@@ -376,7 +376,7 @@ template <int S, bool WIDE>
 static cudaError_t launch_box_t(const DevGeo &g, const BoxCf &c, int n_chains, int ctas, size_t smem, const int8_t *occ,
                                 const double *eci, double *cf, double *energy, cudaStream_t st) {
   auto k = boxcf_kernel<S, WIDE>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k, g);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(n_chains * ctas));

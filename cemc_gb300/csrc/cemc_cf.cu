@@ -257,9 +257,9 @@ __device__ WarpSmem warp_stage(const DevGeo &g, const double *eci, unsigned char
 // from device arrays or as kernel arguments.  Tables too large for the parts use one warp.
 constexpr int kApplyWarps = 8;
 
-int apply_warps(const DevGeo &g, size_t max_smem) {
+int apply_warps(const DevGeo &g) {
   const size_t more = 8 * (size_t)g.n_slots * 32 * kApplyWarps;
-  return warp_layout(g).total + more <= max_smem ? kApplyWarps : 1;
+  return warp_layout(g).total + more <= (size_t)g.max_smem ? kApplyWarps : 1;
 }
 
 template <typename CHANGES>
@@ -465,7 +465,7 @@ cudaError_t launch_recompute(const DevGeo &g, int n_chains, const int8_t *occ, c
   const size_t smem1 =
       align16((size_t)g.n_cols * kCfThreads) + 8 * ((kCfThreads / 32) * (size_t)g.n_eci + (size_t)g.n_bf * g.n_sym);
   auto kern = g.pm1_minus >= 0 ? recompute_partial<true> : recompute_partial<false>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
+  cudaError_t e = allow_smem(kern, g);
   if (e != cudaSuccess) return e;
   kern<<<dim3(nb, n_chains), kCfThreads, smem1, st>>>(g, occ, scratch, nb);
   e = cudaGetLastError();
@@ -474,23 +474,22 @@ cudaError_t launch_recompute(const DevGeo &g, int n_chains, const int8_t *occ, c
   return cudaGetLastError();
 }
 
-// (The bound is the device's, not the launch's: threads with other geometries set the same value.)
 cudaError_t launch_apply(const DevGeo &g, int8_t *occ, double *cf, double *energy, const double *eci, int n,
                          const int32_t *sites, const int8_t *old_sym, const int8_t *new_sym, int32_t *status,
-                         size_t max_smem, cudaStream_t st) {
-  const int nw = apply_warps(g, max_smem);
+                         cudaStream_t st) {
+  const int nw = apply_warps(g);
   const size_t smem = warp_kernel_smem(g) + (nw > 1 ? 8 * (size_t)g.n_slots * 32 * nw : 0);
-  cudaError_t e = cudaFuncSetAttribute(apply_changes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
+  cudaError_t e = allow_smem(apply_changes_kernel, g);
   if (e != cudaSuccess) return e;
   apply_changes_kernel<<<1, 32 * nw, smem, st>>>(g, occ, cf, energy, eci, n, sites, old_sym, new_sym, status);
   return cudaGetLastError();
 }
 
 cudaError_t launch_calculate(const DevGeo &g, int8_t *occ, double *cf, double *energy, const double *eci,
-                             const ChangeArgs &ch, double *out, size_t max_smem, cudaStream_t st) {
-  const int nw = apply_warps(g, max_smem);
+                             const ChangeArgs &ch, double *out, cudaStream_t st) {
+  const int nw = apply_warps(g);
   const size_t smem = warp_kernel_smem(g) + (nw > 1 ? 8 * (size_t)g.n_slots * 32 * nw : 0);
-  cudaError_t e = cudaFuncSetAttribute(calculate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
+  cudaError_t e = allow_smem(calculate_kernel, g);
   if (e != cudaSuccess) return e;
   calculate_kernel<<<1, 32 * nw, smem, st>>>(g, occ, cf, energy, eci, ch, out);
   return cudaGetLastError();
@@ -505,7 +504,7 @@ cudaError_t launch_revert(int n_eci, int8_t *occ, double *cf, double *energy, co
 cudaError_t launch_delta(const DevGeo &g, const int8_t *occ, const double *eci, int move, int sa, int sb, int na,
                          double *de, double *dcf, cudaStream_t st) {
   const size_t smem = warp_kernel_smem(g);
-  cudaError_t e = cudaFuncSetAttribute(delta_e_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(delta_e_kernel, g);
   if (e != cudaSuccess) return e;
   delta_e_kernel<<<1, 32, smem, st>>>(g, occ, eci, move, sa, sb, na, de, dcf);
   return cudaGetLastError();

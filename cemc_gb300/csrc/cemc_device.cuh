@@ -73,6 +73,7 @@ struct DevGeo {
   int box_L, box_nb;
   uint32_t box_mnb, box_mL;    // ceil(2^32 / d) for d = box_nb, box_L (division by multiply-high, checked)
   const uint32_t *box_off;     // [box_nb * n_cols] (dx + 128) | (dy + 128) << 8 | (dz + 128) << 16 | b' << 24
+  int max_smem;  // opt-in shared memory per block of the device
 };
 
 // A neighbour row: in memory (the table, or a row copied to shared memory), or
@@ -397,6 +398,14 @@ __device__ __forceinline__ R site_changes(const DevGeo &g, const uint16_t *terms
   __syncwarp();
   de += eci_changes<R, false, true>(g, lb + 65, lb + 33, kind_s, dec_s, coef_s, part, vb, vb, D, lane, gscale_s[gb]);
   return de;
+}
+
+// A kernel's dynamic shared memory is allowed per function, for all threads of the process: every launch sets the
+// device's bound, not its own size, which another thread's smaller launch could undo between this setting and
+// the launch.
+template <typename K>
+inline cudaError_t allow_smem(K kernel, const DevGeo &g) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, g.max_smem);
 }
 
 }  // namespace cemc

@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(1024, 1) field_kernel(DevGeo g, RunArgs a, Fie
 template <typename R>
 static cudaError_t launch_field_t(const DevGeo &g, const RunArgs &a, const FieldDev &fd, size_t smem, cudaStream_t st) {
   auto k = field_kernel<R>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k, g);
   if (e != cudaSuccess) return e;
   k<<<dim3((unsigned)a.n_chains), dim3((unsigned)field_threads(a.warps)), smem, st>>>(g, a, fd);
   return cudaGetLastError();

@@ -24,9 +24,9 @@ cudaError_t launch_recompute(const DevGeo &g, int n_chains, const int8_t *occ, c
                              double *energy, double *scratch, cudaStream_t st);
 cudaError_t launch_apply(const DevGeo &g, int8_t *occ, double *cf, double *energy, const double *eci, int n,
                          const int32_t *sites, const int8_t *old_sym, const int8_t *new_sym, int32_t *status,
-                         size_t max_smem, cudaStream_t st);
+                         cudaStream_t st);
 cudaError_t launch_calculate(const DevGeo &g, int8_t *occ, double *cf, double *energy, const double *eci,
-                             const ChangeArgs &ch, double *out, size_t max_smem, cudaStream_t st);
+                             const ChangeArgs &ch, double *out, cudaStream_t st);
 cudaError_t launch_revert(int n_eci, int8_t *occ, double *cf, double *energy, const double *snap_cf,
                           const double *snap_energy, const ChangeArgs &ch, cudaStream_t st);
 cudaError_t launch_delta(const DevGeo &g, const int8_t *occ, const double *eci, int move, int sa, int sb, int na,

@@ -1513,7 +1513,7 @@ static cudaError_t launch_t(const DevGeo &g, const RunArgs &a, size_t smem, cuda
   const bool sh = kBoth && a.occ_smem && !a.gstamp && (MOVE == CEMC_MOVE_FLIP || a.trk_smem);
   auto k = sh ? mc_kernel<R, MOVE, FORM, CL, TPW, CONS, kBoth> : mc_kernel<R, MOVE, FORM, CL, TPW, CONS, false>;
   if (block_threads(a) > kMcMaxThreads) return cudaErrorInvalidConfiguration;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k, g);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(a.n_chains * CL));
@@ -1533,9 +1533,9 @@ static cudaError_t launch_t(const DevGeo &g, const RunArgs &a, size_t smem, cuda
 }
 
 template <typename R, int MOVE, int FORM>
-static int clusters_t(const RunArgs &a, size_t smem) {
+static int clusters_t(const DevGeo &g, const RunArgs &a, size_t smem) {
   auto k = mc_kernel<R, MOVE, FORM, 2, 1, false, false>;  // (the same threads, registers bound and memory as its other build)
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
+  if (allow_smem(k, g) != cudaSuccess) return 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(a.n_chains * 2));
   cfg.blockDim = dim3(block_threads(a));
@@ -1596,25 +1596,26 @@ cudaError_t launch_precision(const DevGeo &g, const RunArgs &a, int move, size_t
 }
 
 template <typename R, int FORM>
-static int clusters_m(const RunArgs &a, int move, size_t smem) {
-  return move == CEMC_MOVE_SWAP ? clusters_t<R, CEMC_MOVE_SWAP, FORM>(a, smem) : clusters_t<R, CEMC_MOVE_FLIP, FORM>(a, smem);
+static int clusters_m(const DevGeo &g, const RunArgs &a, int move, size_t smem) {
+  return move == CEMC_MOVE_SWAP ? clusters_t<R, CEMC_MOVE_SWAP, FORM>(g, a, smem)
+                                : clusters_t<R, CEMC_MOVE_FLIP, FORM>(g, a, smem);
 }
 
 template <typename R>
-int clusters_precision(const RunArgs &a, int move, size_t smem, int form) {
-  if (form == kFormSpin) return clusters_m<R, kFormSpin>(a, move, smem);
-  if (form == kFormTable) return clusters_m<R, kFormTable>(a, move, smem);
-  return clusters_m<R, kFormGeneric>(a, move, smem);
+int clusters_precision(const DevGeo &g, const RunArgs &a, int move, size_t smem, int form) {
+  if (form == kFormSpin) return clusters_m<R, kFormSpin>(g, a, move, smem);
+  if (form == kFormTable) return clusters_m<R, kFormTable>(g, a, move, smem);
+  return clusters_m<R, kFormGeneric>(g, a, move, smem);
 }
 
 #ifdef CEMC_MC_F64
 template cudaError_t launch_precision<double>(const DevGeo &, const RunArgs &, int, size_t, cudaStream_t, int,
                                               const SpinDev *);
-template int clusters_precision<double>(const RunArgs &, int, size_t, int);
+template int clusters_precision<double>(const DevGeo &, const RunArgs &, int, size_t, int);
 #else
 extern template cudaError_t launch_precision<double>(const DevGeo &, const RunArgs &, int, size_t, cudaStream_t, int,
                                                      const SpinDev *);
-extern template int clusters_precision<double>(const RunArgs &, int, size_t, int);
+extern template int clusters_precision<double>(const DevGeo &, const RunArgs &, int, size_t, int);
 
 cudaError_t launch_mc(const DevGeo &g, const RunArgs &a, int move, int precision, size_t smem, cudaStream_t st,
                       int form, const SpinDev *spin) {
@@ -1628,9 +1629,9 @@ cudaError_t launch_mc(const DevGeo &g, const RunArgs &a, int move, int precision
                                     : launch_precision<double>(g, a, move, smem, st, form, spin);
 }
 
-int max_active_clusters(const DevGeo &, const RunArgs &a, int move, int precision, size_t smem, int form) {
-  return precision == CEMC_PREC_F32 ? clusters_precision<float>(a, move, smem, form)
-                                    : clusters_precision<double>(a, move, smem, form);
+int max_active_clusters(const DevGeo &g, const RunArgs &a, int move, int precision, size_t smem, int form) {
+  return precision == CEMC_PREC_F32 ? clusters_precision<float>(g, a, move, smem, form)
+                                    : clusters_precision<double>(g, a, move, smem, form);
 }
 #endif
 

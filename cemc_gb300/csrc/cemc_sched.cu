@@ -732,7 +732,7 @@ cudaError_t launch_sched(const DevGeo &g, const RunArgs &a, int precision, size_
   const unsigned threads = (unsigned)((a.warps + kSchedHelpers) * 32);
   if (threads > kSchedMaxThreads || !g.table16 || !sd.qtr_ok) return cudaErrorInvalidConfiguration;
   auto k = precision == CEMC_PREC_F32 ? sched_kernel<float> : sched_kernel<double>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k, g);
   if (e != cudaSuccess) return e;
   k<<<a.n_chains, threads, smem, st>>>(g, a, sd);
   return cudaGetLastError();

@@ -729,7 +729,7 @@ static cudaError_t launch_tick_r(const DevGeo &g, const RunArgs &a, int move, si
   auto k = move != CEMC_MOVE_SWAP ? tick_kernel<R, CEMC_MOVE_FLIP, kTickWarps>
            : a.warps <= kTickWarps ? tick_kernel<R, CEMC_MOVE_SWAP, kTickWarps>
                                    : tick_kernel<R, CEMC_MOVE_SWAP, kTickCap>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k, g);
   if (e != cudaSuccess) return e;
   k<<<a.n_chains, 32 * (a.warps + kTickHelpers), smem, st>>>(g, a);
   return cudaGetLastError();
