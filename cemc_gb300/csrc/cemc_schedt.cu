@@ -493,12 +493,16 @@ __global__ void __launch_bounds__(32 * (WARPS + kTickHelpers), 1) tick_kernel(De
           fin[q] = __ballot_sync(kFull, in && (st & 255u) != 0u);
           acc[q] = __ballot_sync(kFull, in && (st & 255u) != 0u && (st & 256u));
         }
+        // a trial may finish in this very tick: its mask is complete before its state says so (the evaluator's
+        // fence), and is read after it here
+        __threadfence_block();
+        const volatile uint32_t *vmask = mask;
         int done_n = 32, cut = 32;  // trials finished from x0 on, without a gap; first trial touched
 #pragma unroll
         for (int q = 1; q >= 0; --q) {
           const uint32_t x = w0 + 32u * q + lane;
-          uint32_t on = mask[x & rmask] & acc[q];
-          if (q == 1) on |= mask[RG + (x & rmask)] & acc[0];
+          uint32_t on = vmask[x & rmask] & acc[q];
+          if (q == 1) on |= vmask[RG + (x & rmask)] & acc[0];
           const unsigned hit = __ballot_sync(kFull, x >= x0 && x < drawn && on != 0);
           const unsigned gap = __ballot_sync(kFull, x >= x0) & ~fin[q];
           if (hit) cut = (int)(w0 + 32u * q + __ffs(hit) - 1 - x0);
