@@ -612,7 +612,8 @@ def run_gpu(args):
     peak, peak_kind = measured_peak()
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
     busy_sms = min(sms, N_CHAINS * max(1, runner.cluster))
-    ncu_traffic, ncu_ipc, ncu_launch = NCU_FIGURES.get(int(cb.last_kernel), (None, None, None))
+    captured = cb.last_kernel != E.KERNEL_SPIN_QUARTER or cb.last_scheduled  # form 6's figures are the scheduled kernel's
+    ncu_traffic, ncu_ipc, ncu_launch = NCU_FIGURES.get(int(cb.last_kernel) if captured else None, (None, None, None))
 
     # -- end to end through the public batched API, host buffers each step ---------------
     occ_h = torch.from_numpy(occ).pin_memory()
@@ -682,7 +683,7 @@ def run_gpu(args):
                          "traffic_source": NCU_SOURCE + ncu_launch if ncu_launch else None,
                          "peak_kind": peak_kind,
                          "kernel": "field_kernel<float>" if cb.last_kernel == E.KERNEL_FIELD
-                         else "sched_kernel<float>" if cb.last_kernel == E.KERNEL_SPIN_QUARTER
+                         else "sched_kernel<float>" if cb.last_scheduled
                          else "mc_kernel<float, flip, %s>" % KERNEL_NAMES.get(int(cb.last_kernel), ""),
                          "kernel_ms": k_ms,
                          "alg_bytes_per_trial": bytes_per_flip,

@@ -1034,6 +1034,7 @@ int run_sched(const cemc_geometry *geo, cemc_run_desc *r, cemc::RunArgs s, void 
     done += n;
   }
   r->kernel_used = CEMC_KERNEL_SPIN_QUARTER;
+  r->scheduled = 1;
   return CEMC_OK;
 }
 
@@ -1053,6 +1054,7 @@ extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream
     return fail(CEMC_ERR_ARG, "trace buffers must be given together");
   if (r->n_chains > 65535 * 32) return fail(CEMC_ERR_LIMIT, "too many chains in one launch");
   r->kernel_used = CEMC_KERNEL_AUTO;  // nothing launched yet
+  r->scheduled = 0;
   if (r->n_trials == 0) return CEMC_OK;
   if (r->kernel < CEMC_KERNEL_AUTO || r->kernel > CEMC_KERNEL_SPIN_QUARTER)
     return fail(CEMC_ERR_ARG, "unknown kernel %d", (int)r->kernel);
@@ -1345,6 +1347,7 @@ extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream
       if (e != cudaSuccess) return cuda_fail(e, "recompute after the table kernel");
     }
   }
+  r->scheduled = tick_smem ? 1 : 0;
   r->kernel_used = form == cemc::kFormTable ? CEMC_KERNEL_TABLE
                   : (form == cemc::kFormGeneric || form == cemc::kFormRecycle) ? CEMC_KERNEL_GENERIC
                   : (a.tpw == 4 ? CEMC_KERNEL_SPIN_QUARTER : a.tpw == 2 ? CEMC_KERNEL_SPIN_HALFWARP : CEMC_KERNEL_SPIN);

@@ -332,12 +332,13 @@ class ChainBatch:
                          _ptr(chain_trials), int(kernel), int(cluster), _ptr(self.scratch),
                          self.scratch.numel() if self.scratch is not None else 0,
                          _ptr(self._stamps()), self._stamp_buf.numel() if self._stamp_buf is not None else 0,
-                         0, _ptr(site_allow), _ptr(frozen), int(max_attempts), int(bool(accept_first)),
+                         0, 0, _ptr(site_allow), _ptr(frozen), int(max_attempts), int(bool(accept_first)),
                          int(bool(recycle_waste)))
         with torch.cuda.device(self.occ.device):
             _lib.check(self.geo.L.cemc_run(self.geo.handle, C.byref(d), _stream_ptr(self.stream)))
         # the table form ends the call with a full recompute (cf and energy exact already)
         self.last_kernel = int(d.kernel_used)
+        self.last_scheduled = int(d.scheduled)  # a scheduled kernel ran it
         if trace:
             return (tr[0].view(self.n_chains, n_trials, 2), tr[1].view(self.n_chains, n_trials),
                     tr[2].view(self.n_chains, n_trials))
