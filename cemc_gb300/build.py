@@ -10,8 +10,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 SRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT, "libcemc_gb300.so")
-UNITS = ["cemc_mc.cu", "cemc_mc_f64.cu", "cemc_field.cu", "cemc_sched.cu", "cemc_schedt.cu", "cemc_cf.cu", "cemc_boxcf.cu", "cemc_abi.cu"]
-HEADERS = ["cemc_device.cuh", "cemc_launch.h", "cemc_kernels.h", "cemc_spin.h", "cemc_field.h", "cemc_sched.h", "cemc_boxcf.h", "cemc_schedt.h", "cemc_table.cuh", "philox.h"]
+UNITS = ["cemc_mc.cu", "cemc_mc_f64.cu", "cemc_field.cu", "cemc_sched.cu", "cemc_schedt.cu", "cemc_cf.cu", "cemc_boxcf.cu", "cemc_route.cu", "cemc_abi.cu"]
+HEADERS = ["cemc_device.cuh", "cemc_launch.h", "cemc_kernels.h", "cemc_spin.h", "cemc_field.h", "cemc_sched.h", "cemc_boxcf.h", "cemc_schedt.h", "cemc_table.cuh", "cemc_route.h", "philox.h"]
 NVCC_FLAGS = ["-gencode", "arch=compute_103a,code=sm_103a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-O2"]
 

@@ -21,6 +21,7 @@
 #include "cemc_boxcf.h"
 #include "cemc_field.h"
 #include "cemc_kernels.h"
+#include "cemc_route.h"
 #include "cemc_sched.h"
 #include "cemc_schedt.h"
 #include "cemc_spin.h"
@@ -953,7 +954,16 @@ cudaError_t recompute(const cemc_geometry *geo, int n_chains, const int8_t *occ,
   return cemc::launch_recompute(geo->g, n_chains, occ, eci, cf, energy, scratch, st);
 }
 
-// Shape of the scheduled kernel for this geometry, or false where the speculative forms are used.
+// A scheduled kernel for a launch: not at all, for all of its calls, or for those whose chains' state on the device
+// favours it (cemc_route.h).
+struct Scheduled {
+  enum { kNo = 0, kRouted, kAlways } how = kNo;
+  cemc::RunArgs args;
+  cemc::Route route{};
+  size_t smem = 0;
+};
+
+// The scheduled flip kernel for this geometry in booking rounds of `part` trials.
 //
 // Trials that touch one another cannot share a tick: with n_movable / (n_cols + 1) neighbourhoods in the
 // cell, about a third of that many trials can run at once, so small cells take fewer evaluating warps and
@@ -962,27 +972,54 @@ cudaError_t recompute(const cemc_geometry *geo, int n_chains, const int8_t *occ,
 //   2048 sites, 37 neighbourhoods   3.57 / 2.84 / 2.95 / 3.00     864 sites, 16: 4.87 / 6.1 and more
 //   4000 sites, 73                  4.79 / 2.80 / 2.56 / 2.62
 //   16384 sites, 298                5.36 / 3.20 / 2.69 / 2.61     55296 sites, 1005: 8.63 / 6.44 / 5.26 / 4.86
-bool fit_sched(const cemc_geometry *geo, int rsize, int part, cemc::RunArgs &s) {
+//
+// Rounds of chains that accept little are committed nearly whole, while a tick takes its time whatever is
+// accepted, so small cells take this kernel from an acceptance on.  Speculative time over time here, 64 chains,
+// FP32, by the trials of a round and the acceptance:
+//                           0.005  0.08   0.12   0.20   0.28   0.51   0.63   0.70   0.85
+//   37 neighbourhoods   8    0.91          0.96                               1.12   1.17
+//                      16    0.62   0.69   0.72   0.80   0.85   1.03   1.12   1.14   1.23
+//                      18    0.49   0.55   0.59   0.67   0.70   0.87   0.95   0.99   1.08
+//                      32    0.38   0.50   0.57   0.72   0.81   1.09   1.21   1.28   1.40
+//   53                  8    1.20          1.24                               1.38   1.39
+//                      16    0.85   0.92   0.96   1.03   1.09   1.25   1.34   1.36   1.43
+//                      32    0.52   0.65   0.72   0.88   0.97   1.28   1.39   1.46   1.58
+//   72                 16    1.06   1.14   1.16   1.24   1.27   1.41   1.47   1.49   1.55
+//                      32    0.67   0.79   0.86   0.98   1.09   1.38   1.51   1.54   1.67
+//   125                16    1.36   1.44          1.50   1.53   1.60   1.64   1.64   1.65
+//                      32    0.90   1.00   1.07   1.15   1.26   1.48   1.56   1.61   1.70
+//   159                32    1.05   1.15          1.31   1.35   1.54   1.62
+//   1005               32    1.22   1.49          1.59   1.64   1.89   2.06
+//         64, FP32 / FP64    0.85 / 0.82  1.04 / 0.90  1.16 / 0.96  1.22 / 1.00 (acceptance 0.005, 0.08, 0.24, 0.28)
+void fit_sched(const cemc_geometry *geo, int precision, int part, Scheduled &s) {
   const cemc::DevGeo &g = geo->g;
+  const int rsize = precision == CEMC_PREC_F32 ? 4 : 8;
   const int room = g.n_movable / (g.n_cols + 1);
-  if (room < 32) return false;
-  s.warps = room < 64 ? 8 : (room < 128 ? 12 : 16);
-  s.part = part;
+  if (room < 32) return;
+  cemc::RunArgs &a = s.args;
+  a.warps = room < 64 ? 8 : (room < 128 ? 12 : 16);
+  a.part = part;
   int exact = 5;
   while ((1 << exact) < g.n_sites) ++exact;
   // rows of 512 trials cover the eight or so ticks between a row's fetch and the end of its trial; 256
   // (which stalls 12 and 16 warps) where the hash would be left with fewer than 2^13 buckets
-  for (int rows = 9; rows >= 8; --rows) {
-    for (int hb = exact; hb >= (rows == 9 ? std::min(exact, 13) : 8); --hb) {
-      s.row_bits = rows;
-      s.ring_bits = rows + 1;  // a mask's 255 trials before the oldest unfinished one stay in the ring
-      s.head_bits = hb;
-      const size_t need = cemc::sched_layout(g, geo->spin.n_cl, geo->spin.n_masks, rsize, 4 * s.warps, s.ring_bits,
-                                             s.row_bits, s.head_bits).total;
-      if (need <= (size_t)geo->max_smem) return true;
+  for (int rows = 9; rows >= 8 && !s.how; --rows)
+    for (int hb = exact; hb >= (rows == 9 ? std::min(exact, 13) : 8) && !s.how; --hb) {
+      a.row_bits = rows;
+      a.ring_bits = rows + 1;  // a mask's 255 trials before the oldest unfinished one stay in the ring
+      a.head_bits = hb;
+      s.smem = cemc::sched_layout(g, geo->spin.n_cl, geo->spin.n_masks, rsize, 4 * a.warps, a.ring_bits, a.row_bits,
+                                  a.head_bits).total;
+      if (s.smem <= (size_t)geo->max_smem) s.how = Scheduled::kRouted;
     }
-  }
-  return false;
+  if (!s.how) return;
+  if (part <= 8) s.route.hot = room < 48 ? 0.3 : 0.0;
+  else if (part <= 16) s.route.hot = room < 48 ? 0.5 : room < 70 ? 0.2 : 0.0;
+  else if (part <= 32) s.route.hot = room < 48 ? 0.7 : room < 64 ? 0.4 : room < 100 ? 0.25 : room < 150 ? 0.15 : 0.0;
+  else s.route.hot = room < 48 ? 0.7 : room < 64 ? 0.4 : 0.3;
+  if (s.route.hot == 0.0) s.how = Scheduled::kAlways;
+  s.route.share_hot = 0.0;
+  s.route.share = -1.0;
 }
 
 // Shape of the scheduled table kernel, or false where the speculative form is used.
@@ -998,12 +1035,13 @@ bool fit_sched(const cemc_geometry *geo, int rsize, int part, cemc::RunArgs &s) 
 //           18 columns: 1000, 52             0.96 / 1.22 / 1.05            3528, 185  1.24 / 1.77 / 1.25
 // A flip's rows and draws are as cheap ahead in the speculative form, so flips gain only where the evaluation
 // is long, and in FP64 the booking of their singlets (FP64 scans) takes what they gain.
-bool fit_tick(const cemc_geometry *geo, int precision, int move, int part, cemc::RunArgs &s) {
+void fit_tick(const cemc_geometry *geo, int precision, int move, int part, Scheduled &sc) {
   const cemc::DevGeo &g = geo->g;
   const bool swap = move == CEMC_MOVE_SWAP;
   const int room = g.n_movable / ((swap ? 4 : 1) * (g.n_cols + 1));
   const bool wide = g.n_cols >= 48;
-  if (part > 32 || (swap ? room < (wide ? 10 : 40) : (precision != CEMC_PREC_F32 || !wide || room < 40))) return false;
+  if (part > 32 || (swap ? room < (wide ? 10 : 40) : (precision != CEMC_PREC_F32 || !wide || room < 40))) return;
+  cemc::RunArgs &s = sc.args;
   s.part = part;
   s.warps = swap && room < 20 ? 8 : (swap && room >= 150 ? cemc::kTickCap : cemc::kTickWarps);
   int exact = 5;
@@ -1012,30 +1050,12 @@ bool fit_tick(const cemc_geometry *geo, int precision, int move, int part, cemc:
     for (int hb = std::min(exact, 14); hb >= std::min(exact, 11); --hb) {
       s.row_bits = rb;
       s.head_bits = hb;
-      if (cemc::tick_layout(g, swap, precision == CEMC_PREC_F32 ? 4 : 8, rb, hb).total <= (size_t)geo->max_smem)
-        return true;
+      sc.smem = cemc::tick_layout(g, swap, precision == CEMC_PREC_F32 ? 4 : 8, rb, hb).total;
+      if (sc.smem <= (size_t)geo->max_smem) {
+        sc.how = Scheduled::kAlways;
+        return;
+      }
     }
-  return false;
-}
-
-int run_sched(const cemc_geometry *geo, cemc_run_desc *r, cemc::RunArgs s, void *stream) {
-  const cemc::DevGeo &g = geo->g;
-  const size_t smem = cemc::sched_layout(g, geo->spin.n_cl, geo->spin.n_masks, r->precision == CEMC_PREC_F32 ? 4 : 8,
-                                         4 * s.warps, s.ring_bits, s.row_bits, s.head_bits).total;
-  const uint64_t max_chunk = (uint64_t)1 << 25;  // as the speculative forms; trial numbers of a launch fit 32 bits
-  if (r->n_trials > max_chunk && r->trace_acc)
-    return fail(CEMC_ERR_LIMIT, "traced runs are limited to %llu trials per call", (unsigned long long)max_chunk);
-  for (uint64_t done = 0; done < r->n_trials;) {
-    const uint64_t n = std::min(max_chunk, r->n_trials - done);
-    s.n_trials = n;
-    s.chunk_offset = done;
-    cudaError_t e = cemc::launch_sched(g, s, r->precision, smem, static_cast<cudaStream_t>(stream), geo->spin);
-    if (e != cudaSuccess) return cuda_fail(e, "scheduled Monte Carlo kernel launch");
-    done += n;
-  }
-  r->kernel_used = CEMC_KERNEL_SPIN_QUARTER;
-  r->scheduled = 1;
-  return CEMC_OK;
 }
 
 }  // namespace
@@ -1290,14 +1310,18 @@ extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream
     if (!found && r->cluster != 2) found = fit(1, L, a);
   }
   if (!found) return fail(CEMC_ERR_LIMIT, "shared memory exceeds %zu bytes; use fewer warps", budget);
-  // Scheduled kernel: unconstrained spin flips of the automatic and the quarter-warp form.  It books in the
-  // rounds this launch shape would have had with exact conflict tables, so a shape that would hash them stays.
-  if (geo->spin_ok && geo->spin.qtr_ok && g.table16 && form == cemc::kFormSpin && r->move == CEMC_MOVE_FLIP &&
-      !constrained && r->cluster != 2 && (r->kernel == CEMC_KERNEL_AUTO || r->kernel == CEMC_KERNEL_SPIN_QUARTER) &&
-      (a.gstamp || a.stamp_bits == exact_bits)) {
-    cemc::RunArgs s = a;
-    if (fit_sched(geo, rsize, cemc::round_trials(1, a.warps, a.tpw), s)) return run_sched(geo, r, s, stream);
-  }
+  // Scheduled kernels.  They book in the rounds this launch shape would have had with exact conflict tables, so a
+  // shape that would hash them stays.
+  Scheduled sch;
+  sch.args = a;
+  const bool exact = a.gstamp || a.stamp_bits == exact_bits;
+  const bool flips = form == cemc::kFormSpin && r->move == CEMC_MOVE_FLIP;  // else the table form's moves
+  if (flips && geo->spin.qtr_ok && g.table16 && !constrained && exact && r->cluster != 2 &&
+      (r->kernel == CEMC_KERNEL_AUTO || r->kernel == CEMC_KERNEL_SPIN_QUARTER))
+    fit_sched(geo, r->precision, cemc::round_trials(1, a.warps, a.tpw), sch);
+  else if (form == cemc::kFormTable && !constrained && exact)
+    fit_tick(geo, r->precision, r->move, cemc::round_trials(a.cl, a.warps, a.tpw), sch);
+  if (sch.how == Scheduled::kRouted && (!r->status || r->n_trials < cemc::kRouteTrials)) sch.how = Scheduled::kNo;
   // The table form leaves correlation functions to a full recompute at the end of the call.
   double *rscratch = nullptr;
   if (form == cemc::kFormTable) {
@@ -1319,26 +1343,27 @@ extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream
   const uint64_t max_chunk = (uint64_t)1 << 25;
   if (r->n_trials > max_chunk && r->trace_acc)
     return fail(CEMC_ERR_LIMIT, "traced runs are limited to %llu trials per call", (unsigned long long)max_chunk);
-  // Scheduled table kernel: unconstrained moves of the table form, booked in the rounds this launch shape
-  // would have had with exact conflict tables (a shape that would hash them stays).
-  cemc::RunArgs tick = a;
-  size_t tick_smem = 0;
-  if (form == cemc::kFormTable && !constrained && (a.gstamp || a.stamp_bits == exact_bits) &&
-      fit_tick(geo, r->precision, r->move, cemc::round_trials(a.cl, a.warps, a.tpw), tick))
-    tick_smem = cemc::tick_layout(g, is_swap, rsize, tick.row_bits, tick.head_bits).total;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (sch.how == Scheduled::kRouted) {
+    sch.args.route = cemc::kRouteScheduled;
+    a.route = cemc::kRouteSpeculative;
+  }
   for (uint64_t done = 0; done < r->n_trials;) {
     const uint64_t n = std::min(max_chunk, r->n_trials - done);
+    a.n_trials = sch.args.n_trials = n;
+    a.chunk_offset = sch.args.chunk_offset = done;
     cudaError_t e;
-    if (tick_smem) {
-      tick.n_trials = n;
-      tick.chunk_offset = done;
-      e = cemc::launch_tick(g, tick, r->move, r->precision, tick_smem, static_cast<cudaStream_t>(stream));
-      if (e != cudaSuccess) return cuda_fail(e, "scheduled table kernel launch");
-    } else {
-      a.n_trials = n;
-      a.chunk_offset = done;
-      e = cemc::launch_mc(g, a, r->move, r->precision, L.total, static_cast<cudaStream_t>(stream), form,
-                          use_spin ? &geo->spin : nullptr);
+    if (sch.how == Scheduled::kRouted) {
+      e = cemc::launch_route(g, a, is_swap, sch.route, st);
+      if (e != cudaSuccess) return cuda_fail(e, "route kernel launch");
+    }
+    if (sch.how) {
+      e = flips ? cemc::launch_sched(g, sch.args, r->precision, sch.smem, st, geo->spin)
+                : cemc::launch_tick(g, sch.args, r->move, r->precision, sch.smem, st);
+      if (e != cudaSuccess) return cuda_fail(e, "scheduled Monte Carlo kernel launch");
+    }
+    if (sch.how != Scheduled::kAlways) {
+      e = cemc::launch_mc(g, a, r->move, r->precision, L.total, st, form, use_spin ? &geo->spin : nullptr);
       if (e != cudaSuccess) return cuda_fail(e, "Monte Carlo kernel launch");
     }
     done += n;
@@ -1347,10 +1372,10 @@ extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream
       if (e != cudaSuccess) return cuda_fail(e, "recompute after the table kernel");
     }
   }
-  r->scheduled = tick_smem ? 1 : 0;
+  r->scheduled = sch.how == Scheduled::kAlways ? 1 : sch.how == Scheduled::kRouted ? 2 : 0;
   r->kernel_used = form == cemc::kFormTable ? CEMC_KERNEL_TABLE
                   : (form == cemc::kFormGeneric || form == cemc::kFormRecycle) ? CEMC_KERNEL_GENERIC
-                  : (a.tpw == 4 ? CEMC_KERNEL_SPIN_QUARTER : a.tpw == 2 ? CEMC_KERNEL_SPIN_HALFWARP : CEMC_KERNEL_SPIN);
+                  : (a.tpw == 4 || sch.how == Scheduled::kAlways ? CEMC_KERNEL_SPIN_QUARTER : a.tpw == 2 ? CEMC_KERNEL_SPIN_HALFWARP : CEMC_KERNEL_SPIN);
   return CEMC_OK;
 }
 

@@ -40,6 +40,7 @@ struct RunArgs {
   int part;          // scheduled kernel: trials per booking round (the round width of the speculative forms)
   int row_bits;      // scheduled kernel: log2 of the neighbour-row ring (ring_bits: trials in flight)
   int head_bits;     // scheduled kernel: log2 of the site-hash size
+  int route;         // 0, or the mark in a chain's status word that leaves it to this launch (cemc_route.h)
   int cons;          // 1: the build with the constraint redraw loop and first-move acceptance (one CTA per chain)
 };
 

@@ -332,6 +332,7 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
   // A chain with no trials in this launch (an empty serving slot) leaves its
   // state untouched; both CTAs of a pair see the same count and leave together.
   if (a.chain_trials && a.chain_trials[chain] <= a.chunk_offset) return;
+  if (a.route && a.status[chain] != a.route) return;  // left to the other kernel
 
   // ---- prologue: stage tables and the chain's state -------------------------
   for (int k = tid; k < n_eci; k += blockDim.x) {

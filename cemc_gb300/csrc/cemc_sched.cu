@@ -137,6 +137,7 @@ __global__ void __launch_bounds__(kSchedMaxThreads, 1) sched_kernel(DevGeo g, Ru
 
   // A chain with no trials in this launch (an empty serving slot) leaves its state untouched.
   if (a.chain_trials && a.chain_trials[chain] <= a.chunk_offset) return;
+  if (a.route && a.status[chain] != a.route) return;  // left to the other kernel
 
   // ---- prologue ---------------------------------------------------------------
   for (int k = tid; k < n_eci; k += blockDim.x) {

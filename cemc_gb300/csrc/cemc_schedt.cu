@@ -124,6 +124,7 @@ __global__ void __launch_bounds__(32 * (WARPS + kTickHelpers), 1) tick_kernel(De
 
   // A chain with no trials in this launch (an empty serving slot) leaves its state untouched.
   if (a.chain_trials && a.chain_trials[chain] <= a.chunk_offset) return;
+  if (a.route && a.status[chain] != a.route) return;  // left to the other kernel
 
   // ---- prologue ---------------------------------------------------------------
   for (int k = tid; k < n_eci; k += blockDim.x) {

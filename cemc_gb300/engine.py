@@ -338,7 +338,7 @@ class ChainBatch:
             _lib.check(self.geo.L.cemc_run(self.geo.handle, C.byref(d), _stream_ptr(self.stream)))
         # the table form ends the call with a full recompute (cf and energy exact already)
         self.last_kernel = int(d.kernel_used)
-        self.last_scheduled = int(d.scheduled)  # a scheduled kernel ran it
+        self.last_scheduled = int(d.scheduled)  # 1: a scheduled kernel ran it, 2: the device chose
         if trace:
             return (tr[0].view(self.n_chains, n_trials, 2), tr[1].view(self.n_chains, n_trials),
                     tr[2].view(self.n_chains, n_trials))

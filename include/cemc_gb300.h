@@ -180,7 +180,8 @@ typedef struct {
   int32_t kernel_used; /* output: the CEMC_KERNEL_* form cemc_run launched (CEMC_KERNEL_TABLE: the call
                           already ended with a full recompute) */
   int32_t scheduled;   /* output: 1 = the trials ran in a scheduled kernel (trials that do not touch one another in
-                          any order), 0 = in the form kernel_used names.  Same chain, same sums, either way. */
+                          any order), 0 = in the form kernel_used names, 2 = in either, which the acceptance so
+                          far (accum) and the composition decide on the device.  Same chain, same sums, each way. */
   /* Move constraints (mc_constraints.py; redraw loop of montecarlo.py:976-988).  A change (site,
    * old, new) is legal when species `old` is not frozen and species `new` is allowed at `site`;
    * a move is legal when all its changes are.  An illegal proposal is redrawn (draw k of trial t

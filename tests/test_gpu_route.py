@@ -1,0 +1,91 @@
+"""Launches whose kernel the device chooses by the chains' acceptance so far and their composition (cemc_route.cu):
+whatever the running sums say, every chain is run once, by either kernel, to the same bits."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+KB = 8.6173303e-5
+
+
+def _batch(E, L, recipe, species, move, chains, occ=None):
+    from cemc_gb300.lattice import fcc_settings, seeded_ecis
+    from cemc_gb300.tables import CEModel
+    s = fcc_settings(L, *recipe, ["Al", "Mg", "Si"][:species])
+    eci = seeded_ecis(s.cset, 0)
+    m = CEModel(s, list(eci))
+    if occ is None:
+        occ = np.random.default_rng(L).integers(0, species, (chains, m.n_sites)).astype(np.int8)
+    geo = E.Geometry(m)
+    return [E.ChainBatch(geo, occ, m.eci_vector(eci), KB * np.linspace(300.0, 1500.0, chains), move, seed=2)
+            for _ in range(3)]
+
+
+def _counters(E, cb, samples, accepted):
+    cb.accum[:, E.A_NSAMP] = torch.tensor(samples, dtype=torch.int64).view(torch.float64)
+    cb.accum[:, E.A_NACC] = torch.tensor(accepted, dtype=torch.int64).view(torch.float64)
+
+
+def _left(E, cb, samples, accepted):
+    torch.cuda.synchronize()
+    cb.check_status()
+    n = cb.accum[:, E.A_NSAMP:].view(torch.int64).clone()
+    n[:, 0] -= samples
+    n[:, 1] -= accepted
+    out = [cb.occ, cb.cf, cb.energy, cb.trial, cb.accum[:, :E.A_NSAMP], n]
+    return [t.clone() for t in (out + ([cb.trk, cb.loc] if cb.trk is not None else []))]
+
+
+# cells of 8 and 12 evaluating warps, and rounds of more than 32 trials; cold, hot and unknown acceptance
+@pytest.mark.parametrize("L,warps,kernel", [(8, 4, 6), (8, 8, 0), (9, 8, 6), (12, 8, 6), (12, 16, 6)])
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("budgets", [False, True])
+def test_flips_by_acceptance(L, warps, kernel, prec, budgets):
+    from cemc_gb300 import engine as E
+    chains, n = 4, 3001
+    states = [(5000, 0), (5000, 4999), (100, 100)]
+    per = torch.tensor([n, 0, 65, 2999], dtype=torch.int64, device="cuda") if budgets else None
+    got = []
+    for cb, (samples, accepted) in zip(_batch(E, L, (4, 2, 1), 2, E.MOVE_FLIP, chains), states):
+        _counters(E, cb, samples, accepted)
+        for _ in range(2):  # the second call finds the counters of the first
+            cb.run(n, precision=prec, warps=warps, kernel=kernel, cluster=1, chain_trials=per)
+            assert cb.last_scheduled == 2
+        got.append(_left(E, cb, samples, accepted))
+    assert torch.equal(got[0][3], 2 * (per if budgets else torch.full((chains,), n, device="cuda")))
+    for other in got[1:]:
+        for x, y in zip(got[0], other):
+            assert torch.equal(x, y)
+
+
+def test_short_calls_and_calls_without_status_are_not_routed():
+    from cemc_gb300 import engine as E
+    a, b, c = _batch(E, 8, (4, 2, 1), 2, E.MOVE_FLIP, 2)
+    a.run(2047, precision=E.PREC_F32, warps=8, cluster=1)
+    assert a.last_scheduled == 0
+    c.run(2048, precision=E.PREC_F32, warps=8, cluster=1)
+    assert c.last_scheduled == 2
+    b.status = None
+    b.run(3000, precision=E.PREC_F32, warps=8, cluster=1)
+    assert b.last_scheduled == 0
+    torch.cuda.synchronize()
+    assert b.trial.tolist() == [3000, 3000] and c.trial.tolist() == [2048, 2048]
+
+
+def test_routed_launch_in_a_graph():
+    """A captured launch decides anew at each replay; after replays the chain is the one of separate calls."""
+    from cemc_gb300 import engine as E
+    from cemc_gb300.batch import BatchRunner
+    a, _, _ = _batch(E, 8, (4, 2, 1), 2, E.MOVE_FLIP, 3)
+    r = BatchRunner(a.geo, a.occ.cpu().numpy(), a.eci.cpu().numpy(), np.linspace(300.0, 1500.0, 3), E.MOVE_FLIP,
+                    seed=2, warps=8, cluster=1, sweeps_per_step=1.0, recompute_every=1)
+    r.step(4)
+    r.synchronize()
+    assert r.cb.last_scheduled == 2
+    for _ in range(4):
+        a.run(r.trials_per_step, precision=E.PREC_F32, warps=8, cluster=1, kernel=E.KERNEL_SPIN_HALFWARP)
+        a.recompute()
+    torch.cuda.synchronize()
+    for k in ("occ", "cf", "energy", "trial"):
+        assert torch.equal(getattr(a, k), getattr(r.cb, k)), k
