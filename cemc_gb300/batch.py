@@ -163,6 +163,8 @@ class MultiBatchRunner:
         self.stream = torch.cuda.Stream(device=self.device)
         self._graph = None
         self.trials_per_step = sum(r.n_chains * r.trials_per_step for r in self.runners)
+        for r in self.runners:
+            r.cb.beside = self.n_chains - r.n_chains
 
     @property
     def n_chains(self) -> int:

@@ -963,7 +963,8 @@ struct Scheduled {
   size_t smem = 0;
 };
 
-// The scheduled flip kernel for this geometry in booking rounds of `part` trials.
+// The scheduled flip kernel for this geometry in booking rounds of `part` trials, instead of the speculative launch
+// `a` with `smem` bytes and `beside` chains of other launches next to it.
 //
 // Trials that touch one another cannot share a tick: with n_movable / (n_cols + 1) neighbourhoods in the
 // cell, about a third of that many trials can run at once, so small cells take fewer evaluating warps and
@@ -991,12 +992,24 @@ struct Scheduled {
 //   159                32    1.05   1.15          1.31   1.35   1.54   1.62
 //   1005               32    1.22   1.49          1.59   1.64   1.89   2.06
 //         64, FP32 / FP64    0.85 / 0.82  1.04 / 0.90  1.16 / 0.96  1.22 / 1.00 (acceptance 0.005, 0.08, 0.24, 0.28)
-void fit_sched(const cemc_geometry *geo, int precision, int part, Scheduled &s) {
+//
+// One chain takes an SM here.  Two or three CTAs of the speculative forms share one where the cell is small, so with
+// more chains than SMs they are the faster ones, but for wide rounds above 48 neighbourhoods: 200 hot chains, ms,
+// rounds of 8 / 16 / 32 trials, there and here: 2048 sites 1.96 2.96 / 2.12 2.86 / 2.82 2.85, 2916 2.09 2.65 / 2.07
+// 2.46 / 2.70 2.42, 4000 2.06 2.30 / 1.88 2.04 / 2.37 2.00; 6912 (one CTA an SM) 3.99 2.30 / 3.11 1.87 / 2.97 1.74.
+void fit_sched(const cemc_geometry *geo, int precision, int part, size_t smem, int beside, Scheduled &s) {
   const cemc::DevGeo &g = geo->g;
   const int rsize = precision == CEMC_PREC_F32 ? 4 : 8;
   const int room = g.n_movable / (g.n_cols + 1);
   if (room < 32) return;
   cemc::RunArgs &a = s.args;
+  if ((int64_t)a.n_chains + beside > geo->n_sms && room < 150 && (part < 32 || room < 48)) {
+    const auto key = std::make_tuple(a.warps, (int)CEMC_MOVE_FLIP, precision, -a.tpw, smem);
+    std::lock_guard<std::mutex> lock(geo->mu);
+    auto it = geo->pairs.find(key);
+    if (it == geo->pairs.end()) it = geo->pairs.emplace(key, cemc::spin_flip_blocks(g, a, precision, smem)).first;
+    if (it->second > 1) return;
+  }
   a.warps = room < 64 ? 8 : (room < 128 ? 12 : 16);
   a.part = part;
   int exact = 5;
@@ -1318,7 +1331,7 @@ extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream
   const bool flips = form == cemc::kFormSpin && r->move == CEMC_MOVE_FLIP;  // else the table form's moves
   if (flips && geo->spin.qtr_ok && g.table16 && !constrained && exact && r->cluster != 2 &&
       (r->kernel == CEMC_KERNEL_AUTO || r->kernel == CEMC_KERNEL_SPIN_QUARTER))
-    fit_sched(geo, r->precision, cemc::round_trials(1, a.warps, a.tpw), sch);
+    fit_sched(geo, r->precision, cemc::round_trials(1, a.warps, a.tpw), L.total, std::max(0, r->beside), sch);
   else if (form == cemc::kFormTable && !constrained && exact)
     fit_tick(geo, r->precision, r->move, cemc::round_trials(a.cl, a.warps, a.tpw), sch);
   if (sch.how == Scheduled::kRouted && (!r->status || r->n_trials < cemc::kRouteTrials)) sch.how = Scheduled::kNo;

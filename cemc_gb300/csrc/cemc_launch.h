@@ -195,5 +195,7 @@ cudaError_t launch_mc(const DevGeo &g, const RunArgs &a, int move, int precision
                       int form, const SpinDev *spin);
 // Clusters of `cl` CTAs (each with `smem` bytes) that can be resident at once; 0 if none.
 int max_active_clusters(const DevGeo &g, const RunArgs &a, int move, int precision, size_t smem, int form);
+// CTAs of an unconstrained spin-flip launch of two or four trials per warp that share an SM.
+int spin_flip_blocks(const DevGeo &g, const RunArgs &a, int precision, size_t smem);
 
 }  // namespace cemc

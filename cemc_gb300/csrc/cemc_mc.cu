@@ -1533,6 +1533,24 @@ static cudaError_t launch_t(const DevGeo &g, const RunArgs &a, size_t smem, cuda
   return cudaGetLastError();
 }
 
+template <typename R, int TPW>
+static int flip_blocks_t(const DevGeo &g, const RunArgs &a, size_t smem) {
+  auto k = a.occ_smem && !a.gstamp ? mc_kernel<R, CEMC_MOVE_FLIP, kFormSpin, 1, TPW, false, true>
+                                   : mc_kernel<R, CEMC_MOVE_FLIP, kFormSpin, 1, TPW, false, false>;
+  int n = 0;
+  if (allow_smem(k, g) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, (int)block_threads(a), smem) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+
+template <typename R>
+int flip_blocks_precision(const DevGeo &g, const RunArgs &a, size_t smem) {
+  return a.tpw == 4 ? flip_blocks_t<R, 4>(g, a, smem) : flip_blocks_t<R, 2>(g, a, smem);
+}
+
 template <typename R, int MOVE, int FORM>
 static int clusters_t(const DevGeo &g, const RunArgs &a, size_t smem) {
   auto k = mc_kernel<R, MOVE, FORM, 2, 1, false, false>;  // (the same threads, registers bound and memory as its other build)
@@ -1613,10 +1631,12 @@ int clusters_precision(const DevGeo &g, const RunArgs &a, int move, size_t smem,
 template cudaError_t launch_precision<double>(const DevGeo &, const RunArgs &, int, size_t, cudaStream_t, int,
                                               const SpinDev *);
 template int clusters_precision<double>(const DevGeo &, const RunArgs &, int, size_t, int);
+template int flip_blocks_precision<double>(const DevGeo &, const RunArgs &, size_t);
 #else
 extern template cudaError_t launch_precision<double>(const DevGeo &, const RunArgs &, int, size_t, cudaStream_t, int,
                                                      const SpinDev *);
 extern template int clusters_precision<double>(const DevGeo &, const RunArgs &, int, size_t, int);
+extern template int flip_blocks_precision<double>(const DevGeo &, const RunArgs &, size_t);
 
 cudaError_t launch_mc(const DevGeo &g, const RunArgs &a, int move, int precision, size_t smem, cudaStream_t st,
                       int form, const SpinDev *spin) {
@@ -1633,6 +1653,10 @@ cudaError_t launch_mc(const DevGeo &g, const RunArgs &a, int move, int precision
 int max_active_clusters(const DevGeo &g, const RunArgs &a, int move, int precision, size_t smem, int form) {
   return precision == CEMC_PREC_F32 ? clusters_precision<float>(g, a, move, smem, form)
                                     : clusters_precision<double>(g, a, move, smem, form);
+}
+
+int spin_flip_blocks(const DevGeo &g, const RunArgs &a, int precision, size_t smem) {
+  return precision == CEMC_PREC_F32 ? flip_blocks_precision<float>(g, a, smem) : flip_blocks_precision<double>(g, a, smem);
 }
 #endif
 

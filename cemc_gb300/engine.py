@@ -158,6 +158,8 @@ def build_tracker(occ: np.ndarray, n_sym: int, background=None):
 class ChainBatch:
     """State of ``n_chains`` Markov chains of one geometry, resident on the GPU."""
 
+    beside = 0  # chains of other batches that run at the same time (a hint for the choice of kernels)
+
     def __init__(self, geo: Geometry, occ, eci, kT, move: int, seed: int = 0, chain_keys=None,
                  stream: Optional[torch.cuda.Stream] = None):
         self.geo = geo
@@ -333,7 +335,7 @@ class ChainBatch:
                          self.scratch.numel() if self.scratch is not None else 0,
                          _ptr(self._stamps()), self._stamp_buf.numel() if self._stamp_buf is not None else 0,
                          0, 0, _ptr(site_allow), _ptr(frozen), int(max_attempts), int(bool(accept_first)),
-                         int(bool(recycle_waste)))
+                         int(bool(recycle_waste)), int(self.beside))
         with torch.cuda.device(self.occ.device):
             _lib.check(self.geo.L.cemc_run(self.geo.handle, C.byref(d), _stream_ptr(self.stream)))
         # the table form ends the call with a full recompute (cf and energy exact already)

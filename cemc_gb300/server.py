@@ -397,6 +397,7 @@ class MCServer:
         n_max = int(per.max())
         if n_max == 0:
             return False
+        grp.cb.beside = sum(g.active() for g in self.groups.values() if g is not grp)
         with torch.cuda.stream(grp.stream):
             grp.chain_trials.copy_(torch.as_tensor(per), non_blocking=False)
             grp.cb.run(n_max, precision=self.precision, warps=grp.warps, chain_trials=grp.chain_trials,

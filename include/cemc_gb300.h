@@ -195,6 +195,8 @@ typedef struct {
   int32_t recycle_waste;        /* 1: waste recycling (Frenkel 2004; montecarlo.py:937-948): accept when
                                    u > 1 / (1 + exp(-dE / kT)), and every trial adds p0 x (value before) +
                                    p1 x (value of the proposal) to the running sums; generic form, one CTA */
+  int32_t beside;      /* chains of other launches that will share the device with this one; 0 = none.  Only weighs
+                          in the choice between kernels that give the same result */
 } cemc_run_desc;
 
 /* Kernel selection of cemc_run.  AUTO takes the binary spin-basis form when

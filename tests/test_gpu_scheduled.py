@@ -36,3 +36,27 @@ def test_launches_a_scheduled_kernel_takes(L, recipe, species, move, scheduled):
     allow = torch.full((2, m.n_sites), 255, dtype=torch.uint8, device="cuda")
     cb.run(100, precision=E.PREC_F32, warps=8, cluster=1, site_allow=allow)
     assert not cb.last_scheduled
+
+
+def test_more_chains_than_sms_share_them():
+    """Where two CTAs of the speculative form share an SM, more chains than SMs keep it, in one launch or several."""
+    from cemc_gb300 import engine as E
+    from cemc_gb300.batch import BatchRunner, MultiBatchRunner
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+
+    def scheduled(L, chains, beside=0):
+        cb, _ = _batch(E, L, (4, 2, 1), 2, E.MOVE_FLIP, chains)
+        cb.beside = beside
+        cb.run(2100, precision=E.PREC_F32, warps=4, cluster=1)
+        torch.cuda.synchronize()
+        cb.check_status()
+        return cb.last_scheduled
+
+    assert scheduled(8, sms) == 2 and scheduled(8, sms + 1) == 0
+    assert scheduled(8, sms - 9, 9) == 2 and scheduled(8, sms - 9, 10) == 0
+    assert scheduled(14, sms + 1) == 1  # one CTA of either kernel takes an SM
+    cb, m = _batch(E, 8, (4, 2, 1), 2, E.MOVE_FLIP, 3)
+    runners = [BatchRunner(cb.geo, cb.occ.cpu().numpy()[:n], cb.eci.cpu().numpy()[:n], 500.0, E.MOVE_FLIP, warps=4,
+                           cluster=1) for n in (1, 2, 3)]
+    MultiBatchRunner(runners)
+    assert [r.cb.beside for r in runners] == [5, 4, 3]
