@@ -1026,49 +1026,83 @@ void fit_sched(const cemc_geometry *geo, int precision, int part, size_t smem, i
       if (s.smem <= (size_t)geo->max_smem) s.how = Scheduled::kRouted;
     }
   if (!s.how) return;
-  if (part <= 8) s.route.hot = room < 48 ? 0.3 : 0.0;
-  else if (part <= 16) s.route.hot = room < 48 ? 0.5 : room < 70 ? 0.2 : 0.0;
-  else if (part <= 32) s.route.hot = room < 48 ? 0.7 : room < 64 ? 0.4 : room < 100 ? 0.25 : room < 150 ? 0.15 : 0.0;
-  else s.route.hot = room < 48 ? 0.7 : room < 64 ? 0.4 : 0.3;
-  if (s.route.hot == 0.0) s.how = Scheduled::kAlways;
-  s.route.share_hot = 0.0;
-  s.route.share = -1.0;
+  double hot;
+  if (part <= 8) hot = room < 48 ? 0.3 : 0.0;
+  else if (part <= 16) hot = room < 48 ? 0.5 : room < 70 ? 0.2 : 0.0;
+  else if (part <= 32) hot = room < 48 ? 0.7 : room < 64 ? 0.4 : room < 100 ? 0.25 : room < 150 ? 0.15 : 0.0;
+  else hot = room < 48 ? 0.7 : room < 64 ? 0.4 : 0.3;
+  if (hot == 0.0) s.how = Scheduled::kAlways;
+  s.route = {hot, 0.0, 1.0, -1.0, -1.0};
 }
 
-// Shape of the scheduled table kernel, or false where the speculative form is used.
+// The scheduled table kernel for this geometry in booking rounds of `part` trials, instead of the speculative launch
+// in sc.args, with `beside` chains of other launches next to it.
 //
 // `room` is the number of neighbourhoods of a move's sites in the cell; about a third of it can run at once.
-// Measured (ms; speculative form in the default or its best explicit width / here with 8 / 16 / 24 trials a
+// Measured (800 K, ms; speculative form in the default or its best explicit width / here with 8 / 16 / 24 trials a
 // tick; FP32 unless said):
 //   swaps   78 columns: 1372 sites, room 4   4.07 / 4.92 / 5.83 / 7.10     4000, 12   5.93 / 4.44 / 4.90 / 6.17
 //                       16384, 51            4.30 / 2.83 / 2.39 / 2.64     55296, 174 6.03 / 5.55 / 4.27 / 4.24
 //           86 columns: 131072, 376         10.25 / 15.9 / 10.0 / 9.08
-//           18 columns: 1000, 13             2.13 / 2.39 / 2.60            3528, 46   2.71 / 2.58 / 2.22
+//           54 columns: 4000, 18             3.89 / 3.72 / 3.88 / 4.53     16384, 74  4.85 / 3.81 / 3.12 / 3.24
+//           42 columns: 4000, 23             3.65 / 3.41 / 3.37 / 3.95     16384, 95  4.59 / 3.72 / 2.98 / 3.04
+//           18 columns: 1000, 13             2.13 / 2.39 / 2.60            4000, 52   1.98 / 2.18 / 1.92 / 2.03
 //   flips   78 columns: 4000, 50             3.53 / 3.56 / 2.97 (FP64 3.83 / 4.32 / 4.08)
+//           54 columns: 4000, 72             1.94 / 2.28 / 1.75            16384, 297 1.72 / 2.64 / 1.84
+//           42 columns: 4000, 93             1.46 / 1.95 / 1.42            16384, 381 1.58 / 2.57 / 1.77
 //           18 columns: 1000, 52             0.96 / 1.22 / 1.05            3528, 185  1.24 / 1.77 / 1.25
 // A flip's rows and draws are as cheap ahead in the speculative form, so flips gain only where the evaluation
-// is long, and in FP64 the booking of their singlets (FP64 scans) takes what they gain.
-void fit_tick(const cemc_geometry *geo, int precision, int move, int part, Scheduled &sc) {
+// is long, and in FP64 the booking of their singlets (FP64 scans) takes what they gain.  A CTA pair's round of 32 flips
+// beats one SM's ticks in large cells (55296 sites, 54 columns: 2.02 / 2.21).
+//
+// What a tick costs does not depend on what is accepted, but for trials that share a list slot, which run one after
+// the other; see cemc_route.h.  Speculative time over time here by acceptance and by the atoms of the solutes
+// (`share`: probability that two trials share a slot); three species, 78 columns, the lower one of the default shape
+// and of 16 warps, which are CTA pairs unless said:
+//   4000 sites, lists in shared memory    equal parts  0.33: 0.80   0.57: 1.01   0.73: 1.14   0.82: 1.20
+//               two solutes, 256 and 64 atoms each (share 0.0036, 0.014), acceptance 0.85, 0.92: 1.08, 0.88
+//   6912                                  equal parts  0.34: 0.91   0.57: 1.19   0.73: 1.33   0.82: 1.41
+//   16384, lists in device memory         equal parts  0.37: 1.29   0.58: 1.46   0.73: 1.60   0.82: 1.66
+//               one solute, 512, 256, 64, 4 atoms (share 0.0010, 0.0018, 0.0071, 0.11), acceptance 0.24: 1.05, 0.96,
+//                                                     0.71, 0.37;  0.82: 2.10, 1.93, 1.55, 1.16
+//               two solutes, 512, 64, 16 (share 0.0018, 0.014, 0.056), acceptance 0.54, 0.84, 0.95: 1.37, 1.26, 1.06
+//   55296                                 equal parts  0.46: 1.12   0.61: 1.25   0.74: 1.37   0.82: 1.43
+//               one solute, 512, 64, 16, 2 (share 0.0009, 0.0070, 0.028, 0.22), acceptance 0.33: 0.92, 0.72, 0.57,
+//                                                     0.41;  0.82: 1.29, 1.18, 1.04, 0.98
+//   16384, 86 columns, two species, hot, one solute of 256, 32, 2 (share 0.0040, 0.031, 0.50): pairs 2.02, 1.50, 1.47;
+//               one CTA of 16 warps 1.28, 0.86, 0.80, of 8 warps 1.32, 0.78, 0.66
+// Flips, one CTA of 16 warps / the default shape (pairs from 5324 sites): 78 columns 4000 sites 0.003: 0.71 / 0.72,
+// 0.59: 1.01 / 1.04, 0.85: 1.15 / 1.14; 86 columns 6912 sites 0.07: 0.77 / 0.60, 0.67: 0.97 / 1.40, 0.84: 1.03 / 1.64;
+// pairs of 16384 sites, 188 neighbourhoods, 0.67: 1.17, 0.84: 1.32; 55296 sites, conflict tables of one CTA in device
+// memory, 0.24: 1.09 / 0.85, 0.85: 1.18 / 0.99.  Rounds of 8: 1.03 to 1.6, whatever is accepted.
+// Chains on most SMs slow down the smallest swap cells' 8 trials a tick (4000 sites, 78 columns, rounds of 8:
+// 2.42 / 2.37 with 64 chains, 2.49 / 2.76 with 152).
+void fit_tick(const cemc_geometry *geo, int precision, int move, int part, int beside, Scheduled &sc) {
   const cemc::DevGeo &g = geo->g;
+  cemc::RunArgs &s = sc.args;
   const bool swap = move == CEMC_MOVE_SWAP;
   const int room = g.n_movable / ((swap ? 4 : 1) * (g.n_cols + 1));
   const bool wide = g.n_cols >= 48;
   if (part > 32 || (swap ? room < (wide ? 10 : 40) : (precision != CEMC_PREC_F32 || !wide || room < 40))) return;
-  cemc::RunArgs &s = sc.args;
+  if (swap && room < 16 && 2 * ((int64_t)s.n_chains + beside) > geo->n_sms) return;
+  const bool always = !swap && s.cl == 1 && (s.gstamp || part <= 8);
+  if (!swap && !always && room > (s.cl == 2 ? 200 : 128)) return;
+  const bool far_lists = !s.trk_smem;
   s.part = part;
   s.warps = swap && room < 20 ? 8 : (swap && room >= 150 ? cemc::kTickCap : cemc::kTickWarps);
   int exact = 5;
   while ((1 << exact) < g.n_sites) ++exact;
-  for (int rb = 7; rb >= 6; --rb)
-    for (int hb = std::min(exact, 14); hb >= std::min(exact, 11); --hb) {
+  for (int rb = 7; rb >= 6 && !sc.how; --rb)
+    for (int hb = std::min(exact, 14); hb >= std::min(exact, 11) && !sc.how; --hb) {
       s.row_bits = rb;
       s.head_bits = hb;
       sc.smem = cemc::tick_layout(g, swap, precision == CEMC_PREC_F32 ? 4 : 8, rb, hb).total;
-      if (sc.smem <= (size_t)geo->max_smem) {
-        sc.how = Scheduled::kAlways;
-        return;
-      }
+      if (sc.smem <= (size_t)geo->max_smem) sc.how = always ? Scheduled::kAlways : Scheduled::kRouted;
     }
+  if (!swap) sc.route = {s.cl == 2 ? 0.6 : 0.8, 0.0, 1.0, -1.0, -1.0};
+  else if (far_lists && s.cl == 2) sc.route = {0.7, room < 100 ? 1e9 : 0.06, 0.5, 0.008, 0.0008};
+  else if (far_lists) sc.route = {0.7, 0.01, 0.5, 0.004, 0.0008};
+  else sc.route = {0.6, 0.005, 1.0, -1.0, -1.0};
 }
 
 }  // namespace
@@ -1333,7 +1367,7 @@ extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream
       (r->kernel == CEMC_KERNEL_AUTO || r->kernel == CEMC_KERNEL_SPIN_QUARTER))
     fit_sched(geo, r->precision, cemc::round_trials(1, a.warps, a.tpw), L.total, std::max(0, r->beside), sch);
   else if (form == cemc::kFormTable && !constrained && exact)
-    fit_tick(geo, r->precision, r->move, cemc::round_trials(a.cl, a.warps, a.tpw), sch);
+    fit_tick(geo, r->precision, r->move, cemc::round_trials(a.cl, a.warps, a.tpw), std::max(0, r->beside), sch);
   if (sch.how == Scheduled::kRouted && (!r->status || r->n_trials < cemc::kRouteTrials)) sch.how = Scheduled::kNo;
   // The table form leaves correlation functions to a full recompute at the end of the call.
   double *rscratch = nullptr;

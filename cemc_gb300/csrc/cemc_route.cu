@@ -16,13 +16,15 @@
 namespace cemc {
 
 __global__ void route_kernel(RunArgs a, int n_sym, bool swaps, Route q) {
-  bool hot = false, over_hot = false, over = false;
+  bool hot = false, warm = false, over_hot = false, over_warm = false, over = false;
   auto idle = [&](int c) { return a.chain_trials && a.chain_trials[c] <= a.chunk_offset; };
   for (int c = threadIdx.x; c < a.n_chains; c += blockDim.x) {
     if (idle(c)) continue;
     if (a.accum) {
       const cemc_accum *ac = a.accum + (a.accum_slot ? a.accum_slot[c] : c);
-      hot |= ac->n_samples >= kRouteKnown && (double)ac->n_accept >= q.hot * (double)ac->n_samples;
+      const bool known = ac->n_samples >= kRouteKnown;
+      hot |= known && (double)ac->n_accept >= q.hot * (double)ac->n_samples;
+      warm |= known && (double)ac->n_accept >= q.warm * (double)ac->n_samples;
     }
     double share = 0.0;  // probability that two trials draw the same list slot of a species
     if (swaps) {
@@ -35,12 +37,16 @@ __global__ void route_kernel(RunArgs a, int n_sym, bool swaps, Route q) {
       share *= 4.0 / (double)(present * present);  // each species is one of a trial's two with 2 / present
     }
     over_hot |= share > q.share_hot;
+    over_warm |= share > q.share_warm;
     over |= share > q.share;
   }
   hot = __syncthreads_or(hot);
+  warm = __syncthreads_or(warm);
   over_hot = __syncthreads_or(over_hot);
+  over_warm = __syncthreads_or(over_warm);
   over = __syncthreads_or(over);
-  const int32_t mark = (hot && !over_hot) || !over ? kRouteScheduled : kRouteSpeculative;
+  const int32_t mark =
+      (hot && !over_hot) || (warm && !over_warm) || !over ? kRouteScheduled : kRouteSpeculative;
   for (int c = threadIdx.x; c < a.n_chains; c += blockDim.x)
     if (!idle(c)) a.status[c] = mark;
 }

@@ -15,11 +15,11 @@ constexpr uint64_t kRouteTrials = 2048;
 // Trials in a chain's running sums from which its acceptance counts as known.
 constexpr uint64_t kRouteKnown = 1024;
 
-// The chains of a launch take the scheduled kernel when the hottest one accepts at least `hot` of its trials and no
-// chain's trials share a list slot with a probability above `share_hot`, or, whatever is accepted, none above
-// `share`.  (Flips have no list slots: probability 0; a negative bound is never met.)
+// The chains of a launch take the scheduled kernel when no chain's trials share a list slot with a probability above
+// `share`, or `share_warm` if the hottest chain accepts at least `warm` of its trials, or `share_hot` if it
+// accepts `hot`.  (Flips have no list slots: probability 0; a negative bound is never met.)
 struct Route {
-  double hot, share_hot, share;
+  double hot, share_hot, warm, share_warm, share;
 };
 
 cudaError_t launch_route(const DevGeo &g, const RunArgs &a, bool swaps, const Route &q, cudaStream_t st);

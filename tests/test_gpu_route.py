@@ -89,3 +89,69 @@ def test_routed_launch_in_a_graph():
     torch.cuda.synchronize()
     for k in ("occ", "cf", "energy", "trial"):
         assert torch.equal(getattr(a, k), getattr(r.cb, k)), k
+
+
+def _composition(kind, n_sites, species, chains):
+    """Site occupations of `chains` chains; the solutes of `kind` atoms each, or equal parts."""
+    counts = [n_sites // species] * species if kind == "equal" else [0] + [kind] * (species - 1)
+    counts[0] = n_sites - sum(counts[1:])
+    rng = np.random.default_rng(n_sites)
+    return np.stack([rng.permutation(np.repeat(np.arange(species), counts)) for _ in range(chains)]).astype(np.int8)
+
+
+# lists in shared memory (8 trials a tick; 18 columns) and in device memory (16 and 24 a tick); solutes of 1 to 3
+# atoms, of as many as share slots most often in the scheduled kernel (40 and 32), and equal parts
+@pytest.mark.parametrize("L,recipe,species", [(10, (5, 3, 1), 3), (10, (2, 1, 0), 3), (14, (5, 3, 1), 3), (24, (6, 2, 1), 2)])
+@pytest.mark.parametrize("kind", [1, 3, 40, 200, "equal"])
+@pytest.mark.parametrize("prec", [0, 1])
+def test_swaps_by_acceptance_and_composition(L, recipe, species, kind, prec):
+    from cemc_gb300 import engine as E
+    chains, n = 3, 3001
+    n_sites = 4 * L ** 3
+    occ = _composition(kind, n_sites, species, chains)
+    per = torch.tensor([n, 0, 2999], dtype=torch.int64, device="cuda")
+    got = []
+    states = [(5000, 0), (5000, 4999), (100, 100)]
+    for cb, (samples, accepted) in zip(_batch(E, L, recipe, species, E.MOVE_SWAP, chains, occ), states):
+        _counters(E, cb, samples, accepted)
+        for _ in range(2):
+            cb.run(n, precision=prec, warps=8, cluster=1, chain_trials=per)
+            assert cb.last_scheduled == 2
+        got.append(_left(E, cb, samples, accepted))
+    assert torch.equal(got[0][3], 2 * per)
+    for other in got[1:]:
+        for x, y in zip(got[0], other):
+            assert torch.equal(x, y)
+
+
+def _other(E, kind, move):
+    from cemc_gb300.lattice import fcc_settings, hcp_settings, seeded_ecis, with_background
+    from cemc_gb300.tables import CEModel
+    names = ["Al", "Mg", "Si"]
+    s = hcp_settings(16, 8, 2, 1, 1, names) if kind == "hcp" else fcc_settings(10, 5, 3, 1, names)
+    eci = seeded_ecis(s.cset, 0)
+    if kind == "background":
+        s = with_background(s)
+    m = CEModel(s, list(eci))
+    occ = np.random.default_rng(7).integers(0, 3, (2, m.n_sites)).astype(np.int8)
+    if len(m.background):
+        occ[:, m.background] = 0
+    geo = E.Geometry(m)
+    return [E.ChainBatch(geo, occ, m.eci_vector(eci), KB * np.array([400.0, 2000.0]), move, seed=11) for _ in range(2)]
+
+
+@pytest.mark.parametrize("kind,move,prec", [("hcp", 1, 0), ("hcp", 1, 1), ("background", 1, 1), ("background", 0, 1),
+                                            ("fcc", 0, 1)])
+@pytest.mark.parametrize("cluster", [1, 2])
+def test_other_cells_and_flips(kind, move, prec, cluster):
+    """Two translation groups, background sites, flips; rounds of one CTA and of a pair."""
+    from cemc_gb300 import engine as E
+    got = []
+    for cb, accepted in zip(_other(E, kind, move), (0, 5000)):
+        _counters(E, cb, 5000, accepted)
+        for _ in range(2):
+            cb.run(2500, precision=prec, warps=16, cluster=cluster, kernel=E.KERNEL_TABLE)
+            assert cb.last_scheduled == 2
+        got.append(_left(E, cb, 5000, accepted))
+    for x, y in zip(*got):
+        assert torch.equal(x, y)
