@@ -223,18 +223,77 @@ __device__ __forceinline__ int metropolis(R de, uint32_t ua, uint32_t ub, double
   return cemc_u01_53(ua, ub) <= exp(-(double)de / kT);
 }
 
-// The same test of an energy change held as an integer multiple of a quantum (`de` its FP64 value): x =
-// dE/kT is its float conversion times the float quantum / kT, two roundings more than above.
-template <typename R>
-__device__ __forceinline__ int metropolis_fx(long long de_fx, R de, uint32_t ua, uint32_t ub, double kT, float q_kT) {
-  if (de_fx < 0) return 1;
-  const float x = (float)de_fx * q_kT;
+// FP64 launches hold ECI coefficients as fixed-point numbers of 64 + kFxLow bits: this part's FP64 pipe issues one
+// warp instruction in 16 cycles per SM, so FP64 additions of an energy change in each of 16 warps cost more than the
+// rest of a round, while integer additions go through the wide pipe, and are exact.  A number is hi + lo 2^-kFxLow
+// quanta, lo counted up from zero, so that the sign of a sum is that of its hi once lo is carried over.
+constexpr int kFxLow = 20;
+constexpr uint32_t kFxMask = (1u << kFxLow) - 1u;
+constexpr int kFxTerms = 1 << (30 - kFxLow);  // factors of fx_mul are smaller: its low product fits 32 bits
+struct FxNum {
+  long long hi;
+  uint32_t lo;  // at most 2^kFxLow
+};
+// Quanta per unit (a power of two) for sums of magnitude up to `bound`, or 0 where FP64 arithmetic stays: for
+// infinite or NaN coefficients, and where `least`, the smallest nonzero one, would not be held to the last of its 53
+// bits.  A sum of such numbers has no rounding at all, so it is never further off than the FP64 sum.  `bound` is
+// about 2^9 times the largest coefficient (as many terms), so coefficients may span a factor of about 2^20.
+__device__ __forceinline__ double fx_quanta(double bound, double least) {
+  if (!(bound < 1e300)) return 0.0;
+  if (!(bound > 1e-200)) return bound == 0.0 ? 1.0 : 0.0;
+  const double scale = ldexp(1.0, 61 - ilogb(bound));  // sums stay below 2^62
+  return least * scale >= ldexp(1.0, 53 - kFxLow) ? scale : 0.0;
+}
+__device__ __forceinline__ FxNum fx_of(double v, double scale) {
+  const double x = v * scale;
+  FxNum f;
+  f.hi = __double2ll_rd(x);
+  f.lo = __double2uint_rn((x - (double)f.hi) * (double)(1u << kFxLow));
+  return f;
+}
+__device__ __forceinline__ FxNum fx_carry(long long hi, int lo) {
+  return FxNum{hi + (long long)(lo >> kFxLow), (uint32_t)lo & kFxMask};
+}
+// f times n, |n| below kFxTerms.
+__device__ __forceinline__ FxNum fx_mul(FxNum f, int n) { return fx_carry(f.hi * (long long)n, (int)f.lo * n); }
+// Sum over each group of LW lanes, plus `c`, times `delta` (+-2).
+template <int LW>
+__device__ __forceinline__ FxNum fx_sum(FxNum f, FxNum c, int delta) {
+  if constexpr (LW == 32) {
+    f.lo = __reduce_add_sync(kFull, f.lo);
+  } else {
+#pragma unroll
+    for (int o = LW / 2; o > 0; o >>= 1) f.lo += __shfl_xor_sync(kFull, f.lo, o);
+  }
+#pragma unroll
+  for (int o = LW / 2; o > 0; o >>= 1) f.hi += __shfl_xor_sync(kFull, f.hi, o);
+  return fx_mul(FxNum{f.hi + c.hi, f.lo + c.lo}, delta);
+}
+// Its FP64 value, rounded to nearest, put together by integer instructions: a conversion and a product on the FP64
+// pipe take longer (half-warp flips of 64 x 16384 sites 5.69 ms with them, 5.44 without).  inv: units per quantum.
+__device__ __forceinline__ double fx_value(FxNum f, double inv) {
+  const int h = (int)(f.hi >> 32);
+  const int s = min(kFxLow, max(0, __clz(h ^ (h >> 31)) - 2));
+  const long long m = (long long)((unsigned long long)f.hi << s) | (long long)(f.lo >> (kFxLow - s));  // in 2^-s quanta
+  unsigned long long u = (unsigned long long)(m < 0 ? -m : m);
+  const int z = __clzll((long long)u);
+  u <<= z & 63;
+  const uint32_t e = (uint32_t)__double2hiint(inv) + ((uint32_t)(62 - z - s) << 20);  // exponent, less the leading bit
+  const unsigned long long d = (u >> 11) + ((u >> 10) & 1u) + ((unsigned long long)e << 32);
+  return z == 64 ? 0.0 : __longlong_as_double((long long)(d | ((unsigned long long)m & 0x8000000000000000ull)));
+}
+
+// The same test of an energy change in fixed point: x = dE/kT is its float conversion times the float quantum / kT,
+// two roundings more than above.
+__device__ __forceinline__ int metropolis_fx(FxNum de, double de_value, uint32_t ua, uint32_t ub, double kT, float q_kT) {
+  if (de.hi < 0) return 1;
+  const float x = (float)de.hi * q_kT;
   const float uf = (float)ua * 2.3283064e-10f;  // a * 2^-32
   const float y = __logf(uf) + x;
   const float margin = 1e-4f + 1e-6f * x + 1e-8f / uf;  // uf == 0 gives an infinite margin
   if (y < -margin) return 1;
   if (y > margin) return 0;
-  return cemc_u01_53(ua, ub) <= exp(-(double)de / kT);
+  return cemc_u01_53(ua, ub) <= exp(-de_value / kT);
 }
 
 // The same test with the uniform's parts precomputed (by the fetcher, off the
@@ -252,16 +311,15 @@ __device__ __forceinline__ int metropolis_pre(R de, float lnu, float mu, const u
   if (yes || y > margin) return yes;  // one branch, almost always taken
   return cemc_u01_53(uw[0], uw[1]) <= exp(-(double)de / kT);
 }
-// metropolis_pre() of an energy change held as an integer multiple of a quantum (see metropolis_fx).
-template <typename R>
-__device__ __forceinline__ int metropolis_pre_fx(long long de_fx, R de, float lnu, float mu, const uint32_t *uw,
+// metropolis_pre() of an energy change in fixed point (see metropolis_fx).
+__device__ __forceinline__ int metropolis_pre_fx(FxNum de, double de_value, float lnu, float mu, const uint32_t *uw,
                                                  double kT, float q_kT) {
-  const float x = (float)de_fx * q_kT;
+  const float x = (float)de.hi * q_kT;
   const float y = lnu + x;
   const float margin = mu + 1e-6f * x;  // u == 0 gives an infinite margin
-  const bool yes = de_fx < 0 || y < -margin;
+  const bool yes = de.hi < 0 || y < -margin;
   if (yes || y > margin) return yes;
-  return cemc_u01_53(uw[0], uw[1]) <= exp(-(double)de / kT);
+  return cemc_u01_53(uw[0], uw[1]) <= exp(-de_value / kT);
 }
 __device__ __forceinline__ void metropolis_parts(uint32_t ua, float &lnu, float &mu) {
   const float uf = (float)ua * 2.3283064e-10f;  // a * 2^-32

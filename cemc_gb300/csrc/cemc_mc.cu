@@ -771,7 +771,7 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
   // spin path: lane k of every evaluating warp holds cluster ECI k and its coefficient
   SpinEci sp_e{};
   R sp_coef = (R)0;
-  long long sp_cfx = 0, sing_fx = 0;  // FP64: the coefficients in units of fx_inv
+  FxNum sp_cfx{0, 0u}, sing_fx{0, 0u};  // FP64: the coefficients in units of fx_inv
   constexpr bool SFX = SPIN && sizeof(R) == 8;
   unsigned sp_multi = 0;  // cluster ECIs with multi-site terms
   // Flips at one or two trials per warp: the odd-term counts of all multi-site ECIs by one
@@ -795,12 +795,18 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
       const double own = lane < 32 / TPW ? (SWAP ? 4.0 : 2.0) * fabs((double)sp_coef) * (double)(sp_e.n_pairs + sp_e.n_multi)
                                          : 0.0;
       const double sing = sd.singlet_eci >= 0 && !SWAP ? (double)coef_s[sd.singlet_eci] : 0.0;
-      fx_scale = fixed_point_scale(warp_sum(own) + 2.0 * fabs(sing), 0);
+      double least = HUGE_VAL;  // smallest nonzero coefficient
+      if (lane < 32 / TPW && (double)sp_coef != 0.0) least = fabs((double)sp_coef);
+      if (sing != 0.0) least = fmin(least, fabs(sing));
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) least = fmin(least, __shfl_xor_sync(kFull, least, o));
+      fx_scale = fx_quanta(warp_sum(own) + 2.0 * fabs(sing), least);
+      if (__any_sync(kFull, (SWAP ? 2 : 1) * (sp_e.n_pairs + sp_e.n_multi) >= kFxTerms)) fx_scale = 0.0;
       if (fx_scale != 0.0) {
         fx_inv = 1.0 / fx_scale;
         fx_kT = (float)(fx_inv / kT);
-        sp_cfx = __double2ll_rn((double)sp_coef * fx_scale);
-        sing_fx = __double2ll_rn(sing * fx_scale);
+        sp_cfx = fx_of((double)sp_coef, fx_scale);
+        sing_fx = fx_of(sing, fx_scale);
       }
     }
     sp_multi = __ballot_sync(kFull, el < sd.n_cl && sp_e.n_multi > 0);
@@ -1031,14 +1037,11 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
                         2 * (__popc(wl & sp_e.pair_lo) + __popc(wh & sp_e.pair_hi) + (hl < sd.n_cl ? my_odd : 0));
           if (hl < sd.n_cl && has) Dh[sp_e.eci] = delta * P;
           R de;
-          long long de_fx = 0;
+          FxNum de_fx{0, 0u};
           if (SFX && fx_scale != 0.0) {
             if (sd.singlet_eci >= 0 && hl == 0 && has) Dh[sd.singlet_eci] = delta;
-            long long sum = sp_cfx * (long long)P;
-#pragma unroll
-            for (int o = LW / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
-            de_fx = (sum + sing_fx) * (long long)delta;
-            de = (R)((double)de_fx * fx_inv);
+            de_fx = fx_sum<LW>(fx_mul(sp_cfx, P), sing_fx, delta);
+            de = (R)fx_value(de_fx, fx_inv);
           } else {
             R sum = sp_coef * (R)P;
 #pragma unroll
@@ -1052,7 +1055,7 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
           // every lane of the group has the trial's energy change and makes its test
           int acc = 0;
           if (has)
-            acc = SFX && fx_scale != 0.0 ? metropolis_pre_fx(de_fx, de, lnu, mu, &draws[slot].x0, kT, fx_kT)
+            acc = SFX && fx_scale != 0.0 ? metropolis_pre_fx(de_fx, (double)de, lnu, mu, &draws[slot].x0, kT, fx_kT)
                                          : metropolis_pre<R>(de, lnu, mu, &draws[slot].x0, kT, inv_kT);
           if (hl == 0 && has) {
             put(&r_sa[gh], (int32_t)sa);
@@ -1181,7 +1184,7 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
               gb = g.site_group[sb];
             }
           }
-          long long de_fx = 0;  // the energy change in units of fx_inv
+          FxNum de_fx{0, 0u};  // the energy change in units of fx_inv
           if constexpr (TAB) {
             __syncwarp();
             const int S = g.n_sym;
@@ -1201,9 +1204,9 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
                                                                            gstart_s[gb], gstart_s[gb + 1], lane);
             };
             if (FX && fx_scale != 0.0) {
-              de_fx = change(ftab_fx);
-              if (!SWAP) de_fx += sfx_s[old_a * S + na];
-              de = (R)((double)de_fx * fx_inv);
+              de_fx.hi = change(ftab_fx);
+              if (!SWAP) de_fx.hi += sfx_s[old_a * S + na];
+              de = (R)((double)de_fx.hi * fx_inv);
             } else {
               de = change(ftab);
               if (!SWAP)
@@ -1263,11 +1266,8 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
             }
             if (sd.singlet_eci >= 0 && lane == 0) Dw[sd.singlet_eci] = SWAP ? 0 : delta;
             if (SFX && fx_scale != 0.0) {
-              long long sum = sp_cfx * (long long)P;
-#pragma unroll
-              for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
-              de_fx = (sum + sing_fx) * (long long)delta;
-              de = (R)((double)de_fx * fx_inv);
+              de_fx = fx_sum<32>(fx_mul(sp_cfx, P), SWAP ? FxNum{0, 0u} : sing_fx, delta);
+              de = (R)fx_value(de_fx, fx_inv);
             } else {
               R sum = warp_sum(sp_coef * (R)P);
               if (sd.singlet_eci >= 0 && !SWAP) sum += coef_s[sd.singlet_eci];
@@ -1284,12 +1284,12 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
               const float lnu = __uint_as_float(SWAP ? (uint32_t)dr.site : dr.x0);
               const float mu = __uint_as_float(SWAP ? dr.pad : dr.x1);
               const uint32_t *uw = SWAP ? &draws[slot].x0 : &draws[slot].w2;
-              acc = (FX || SFX) && fx_scale != 0.0 ? metropolis_pre_fx(de_fx, de, lnu, mu, uw, kT, fx_kT)
+              acc = (FX || SFX) && fx_scale != 0.0 ? metropolis_pre_fx(de_fx, (double)de, lnu, mu, uw, kT, fx_kT)
                                                    : metropolis_pre<R>(de, lnu, mu, uw, kT, inv_kT);
             } else {
               acc = no_move ? 0
                             : (first ? 1
-                                     : ((FX || SFX) && fx_scale != 0.0 ? metropolis_fx(de_fx, de, ua, ub, kT, fx_kT)
+                                     : ((FX || SFX) && fx_scale != 0.0 ? metropolis_fx(de_fx, (double)de, ua, ub, kT, fx_kT)
                                                               : metropolis<R>(de, ua, ub, kT, inv_kT)));
             }
             if (CONS && no_move) put(&misc[3], 1);  // reported in the status at the end of the launch

@@ -229,19 +229,23 @@ __global__ void __launch_bounds__(kSchedMaxThreads, 1) sched_kernel(DevGeo g, Ru
       ms[i] = m.z;
     }
     const R sing = sd.singlet_eci >= 0 ? coef_s[sd.singlet_eci] : (R)0;
-    constexpr bool FX = sizeof(R) == 8;  // FP64: energy changes in fixed point (fixed_point_scale)
+    constexpr bool FX = sizeof(R) == 8;  // FP64: energy changes in fixed point (fx_quanta)
     double fx_inv = 0.0;                 // their quantum, 0: FP64 arithmetic
     float fx_kT = 0.f;
-    long long coef_fx = 0, sing_fx = 0;
+    FxNum coef_fx{0, 0u}, sing_fx{0, 0u};
     if constexpr (FX) {
       // |P| is at most the ECI's terms, the spin change 2
       const double most = warp_sum(lane < 8 ? 2.0 * fabs((double)coef) * (double)p_all : 0.0) + 2.0 * fabs((double)sing);
-      const double scale = fixed_point_scale(most, 0);
+      double least = lane < 8 && (double)coef != 0.0 ? fabs((double)coef) : HUGE_VAL;  // smallest nonzero coefficient
+      if ((double)sing != 0.0) least = fmin(least, fabs((double)sing));
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) least = fmin(least, __shfl_xor_sync(kFull, least, o));
+      const double scale = fx_quanta(most, least);
       if (scale != 0.0) {
         fx_inv = 1.0 / scale;
         fx_kT = (float)(fx_inv / kT);
-        coef_fx = __double2ll_rn((double)coef * scale);
-        sing_fx = __double2ll_rn((double)sing * scale);
+        coef_fx = fx_of((double)coef, scale);
+        sing_fx = fx_of((double)sing, scale);
       }
     }
     const bool cols = 8 * hl < cp16;  // this lane's eight columns 8 hl .. 8 hl + 7 of a row
@@ -331,13 +335,10 @@ __global__ void __launch_bounds__(kSchedMaxThreads, 1) sched_kernel(DevGeo g, Ru
         const int P = p_all - 2 * (__popc(wl & se.pair_lo) + __popc(wh & se.pair_hi) + my_odd);
         const int delta = ((uint32_t)oa ^ xorv) ? 2 : -2;
         R de;
-        long long de_fx = 0;
+        FxNum de_fx{0, 0u};
         if (FX && fx_inv != 0.0) {
-          long long sum = coef_fx * (long long)P;
-#pragma unroll
-          for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
-          de_fx = (sum + sing_fx) * (long long)delta;
-          de = (R)((double)de_fx * fx_inv);
+          de_fx = fx_sum<8>(fx_mul(coef_fx, P), sing_fx, delta);
+          de = (R)fx_value(de_fx, fx_inv);
         } else {
           R sum = coef * (R)P;
 #pragma unroll
@@ -348,7 +349,7 @@ __global__ void __launch_bounds__(kSchedMaxThreads, 1) sched_kernel(DevGeo g, Ru
         int acc = 0;
         if (hl == 0 && has) {
           const float lnu = __uint_as_float(dr.y), mu = __uint_as_float(dr.z);
-          acc = FX && fx_inv != 0.0 ? metropolis_pre_fx(de_fx, de, lnu, mu, &uni[slot].x, kT, fx_kT)
+          acc = FX && fx_inv != 0.0 ? metropolis_pre_fx(de_fx, (double)de, lnu, mu, &uni[slot].x, kT, fx_kT)
                                     : metropolis_pre<R>(de, lnu, mu, &uni[slot].x, kT, inv_kT);
           const int na = oa ^ 1;
           if (acc) occ[sa] = (int8_t)na;

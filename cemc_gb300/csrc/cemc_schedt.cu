@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(32 * (WARPS + kTickHelpers), 1) tick_kernel(De
                   de += coef_s[g.singlet_eci[b]] * (bf_s[b * S + na] - bf_s[b * S + oa]);
           }
           if (lane == 0) {
-            const int acc = FX && fx_scale != 0.0 ? metropolis_fx(de_fx, de, d.ua, d.ub, kT, fx_kT)
+            const int acc = FX && fx_scale != 0.0 ? metropolis_fx(FxNum{de_fx, 0u}, (double)de, d.ua, d.ub, kT, fx_kT)
                                                   : metropolis<R>(de, d.ua, d.ub, kT, inv_kT);
             if (acc) {
               occ[sa] = (int8_t)na;
