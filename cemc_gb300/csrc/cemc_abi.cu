@@ -1092,13 +1092,16 @@ void fit_tick(const cemc_geometry *geo, int precision, int move, int part, int b
   s.warps = swap && room < 20 ? 8 : (swap && room >= 150 ? cemc::kTickCap : cemc::kTickWarps);
   int exact = 5;
   while ((1 << exact) < g.n_sites) ++exact;
-  for (int rb = 7; rb >= 6 && !sc.how; --rb)
-    for (int hb = std::min(exact, 14); hb >= std::min(exact, 11) && !sc.how; --hb) {
-      s.row_bits = rb;
-      s.head_bits = hb;
-      sc.smem = cemc::tick_layout(g, swap, precision == CEMC_PREC_F32 ? 4 : 8, rb, hb).total;
-      if (sc.smem <= (size_t)geo->max_smem) sc.how = always ? Scheduled::kAlways : Scheduled::kRouted;
-    }
+  for (; s.fx_low >= 0 && !sc.how; --s.fx_low)
+    for (int rb = 7; rb >= 6 && !sc.how; --rb)
+      for (int hb = std::min(exact, 14); hb >= std::min(exact, 11) && !sc.how; --hb) {
+        s.row_bits = rb;
+        s.head_bits = hb;
+        sc.smem = cemc::tick_layout(g, swap, precision == CEMC_PREC_F32 ? 4 : 8, rb, hb).total +
+                  (s.fx_low ? cemc::fx_low_bytes(g) : 0);
+        if (sc.smem <= (size_t)geo->max_smem) sc.how = always ? Scheduled::kAlways : Scheduled::kRouted;
+      }
+  ++s.fx_low;  // as it was when the shape was found
   if (!swap) sc.route = {s.cl == 2 ? 0.6 : 0.8, 0.0, 1.0, -1.0, -1.0};
   else if (far_lists && s.cl == 2) sc.route = {0.7, room < 100 ? 1e9 : 0.06, 0.5, 0.008, 0.0008};
   else if (far_lists) sc.route = {0.7, 0.01, 0.5, 0.004, 0.0008};
@@ -1359,6 +1362,8 @@ extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream
   if (!found) return fail(CEMC_ERR_LIMIT, "shared memory exceeds %zu bytes; use fewer warps", budget);
   // Scheduled kernels.  They book in the rounds this launch shape would have had with exact conflict tables, so a
   // shape that would hash them stays.
+  // FP64 table entries in fixed point where there is room for their low parts, in both kernels or in none.
+  if (form == cemc::kFormTable && r->precision == CEMC_PREC_F64) a.fx_low = L.total + cemc::fx_low_bytes(g) <= budget;
   Scheduled sch;
   sch.args = a;
   const bool exact = a.gstamp || a.stamp_bits == exact_bits;
@@ -1391,6 +1396,8 @@ extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream
   if (r->n_trials > max_chunk && r->trace_acc)
     return fail(CEMC_ERR_LIMIT, "traced runs are limited to %llu trials per call", (unsigned long long)max_chunk);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (sch.how) a.fx_low = sch.args.fx_low;
+  const size_t mc_smem = L.total + (a.fx_low ? cemc::fx_low_bytes(g) : 0);
   if (sch.how == Scheduled::kRouted) {
     sch.args.route = cemc::kRouteScheduled;
     a.route = cemc::kRouteSpeculative;
@@ -1410,7 +1417,7 @@ extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream
       if (e != cudaSuccess) return cuda_fail(e, "scheduled Monte Carlo kernel launch");
     }
     if (sch.how != Scheduled::kAlways) {
-      e = cemc::launch_mc(g, a, r->move, r->precision, L.total, st, form, use_spin ? &geo->spin : nullptr);
+      e = cemc::launch_mc(g, a, r->move, r->precision, mc_smem, st, form, use_spin ? &geo->spin : nullptr);
       if (e != cudaSuccess) return cuda_fail(e, "Monte Carlo kernel launch");
     }
     done += n;

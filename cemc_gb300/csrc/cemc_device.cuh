@@ -223,39 +223,45 @@ __device__ __forceinline__ int metropolis(R de, uint32_t ua, uint32_t ub, double
   return cemc_u01_53(ua, ub) <= exp(-(double)de / kT);
 }
 
-// FP64 launches hold ECI coefficients as fixed-point numbers of 64 + kFxLow bits: this part's FP64 pipe issues one
-// warp instruction in 16 cycles per SM, so FP64 additions of an energy change in each of 16 warps cost more than the
-// rest of a round, while integer additions go through the wide pipe, and are exact.  A number is hi + lo 2^-kFxLow
-// quanta, lo counted up from zero, so that the sign of a sum is that of its hi once lo is carried over.
-constexpr int kFxLow = 20;
-constexpr uint32_t kFxMask = (1u << kFxLow) - 1u;
-constexpr int kFxTerms = 1 << (30 - kFxLow);  // factors of fx_mul are smaller: its low product fits 32 bits
+// FP64 launches hold ECI coefficients (spin forms) and table entries as fixed-point numbers of 64 + LOW bits: this
+// part's FP64 pipe issues one warp instruction in 16 cycles per SM, so FP64 additions of an energy change in each of
+// 16 warps cost more than the rest of a round, while integer additions go through the wide pipe, and are exact.  A
+// number is hi + lo 2^-LOW quanta, lo counted up from zero, so that the sign of a sum is that of its hi once lo is
+// carried over.
+constexpr int kFxLow = 20;      // spin forms: their low products fit 32 bits
+constexpr int kFxTableLow = 24;  // table entries: 128 of them a lane are added without a carry
+constexpr int kFxTerms = 1 << (30 - kFxLow);  // factors of fx_mul are smaller
 struct FxNum {
   long long hi;
-  uint32_t lo;  // at most 2^kFxLow
+  uint32_t lo;  // at most 2^LOW
 };
 // Quanta per unit (a power of two) for sums of magnitude up to `bound`, or 0 where FP64 arithmetic stays: for
-// infinite or NaN coefficients, and where `least`, the smallest nonzero one, would not be held to the last of its 53
-// bits.  A sum of such numbers has no rounding at all, so it is never further off than the FP64 sum.  `bound` is
-// about 2^9 times the largest coefficient (as many terms), so coefficients may span a factor of about 2^20.
+// infinite or NaN coefficients, and where the low bits would not reach the last of the 53 bits of `least`, the smallest
+// nonzero coefficient.  Coefficients are held as they are, and a sum of such numbers has no rounding at all, so it is
+// never further off than the FP64 sum; table entries, sums of products of coefficients that are rounded themselves,
+// are rounded by at most half the spacing of FP64 numbers at the smallest coefficient.  `bound` is about 2^9 (as many
+// terms) times the largest coefficient or entry, so coefficients may span a factor of 2^20 (spin) or 2^17 (tables).
+template <int LOW>
 __device__ __forceinline__ double fx_quanta(double bound, double least) {
   if (!(bound < 1e300)) return 0.0;
   if (!(bound > 1e-200)) return bound == 0.0 ? 1.0 : 0.0;
   const double scale = ldexp(1.0, 61 - ilogb(bound));  // sums stay below 2^62
-  return least * scale >= ldexp(1.0, 53 - kFxLow) ? scale : 0.0;
+  return least * scale >= ldexp(1.0, 53 - LOW) ? scale : 0.0;
 }
+template <int LOW>
 __device__ __forceinline__ FxNum fx_of(double v, double scale) {
   const double x = v * scale;
   FxNum f;
   f.hi = __double2ll_rd(x);
-  f.lo = __double2uint_rn((x - (double)f.hi) * (double)(1u << kFxLow));
+  f.lo = __double2uint_rn((x - (double)f.hi) * (double)(1u << LOW));
   return f;
 }
+template <int LOW>
 __device__ __forceinline__ FxNum fx_carry(long long hi, int lo) {
-  return FxNum{hi + (long long)(lo >> kFxLow), (uint32_t)lo & kFxMask};
+  return FxNum{hi + (long long)(lo >> LOW), (uint32_t)lo & ((1u << LOW) - 1u)};
 }
 // f times n, |n| below kFxTerms.
-__device__ __forceinline__ FxNum fx_mul(FxNum f, int n) { return fx_carry(f.hi * (long long)n, (int)f.lo * n); }
+__device__ __forceinline__ FxNum fx_mul(FxNum f, int n) { return fx_carry<kFxLow>(f.hi * (long long)n, (int)f.lo * n); }
 // Sum over each group of LW lanes, plus `c`, times `delta` (+-2).
 template <int LW>
 __device__ __forceinline__ FxNum fx_sum(FxNum f, FxNum c, int delta) {
@@ -271,10 +277,11 @@ __device__ __forceinline__ FxNum fx_sum(FxNum f, FxNum c, int delta) {
 }
 // Its FP64 value, rounded to nearest, put together by integer instructions: a conversion and a product on the FP64
 // pipe take longer (half-warp flips of 64 x 16384 sites 5.69 ms with them, 5.44 without).  inv: units per quantum.
+template <int LOW>
 __device__ __forceinline__ double fx_value(FxNum f, double inv) {
   const int h = (int)(f.hi >> 32);
-  const int s = min(kFxLow, max(0, __clz(h ^ (h >> 31)) - 2));
-  const long long m = (long long)((unsigned long long)f.hi << s) | (long long)(f.lo >> (kFxLow - s));  // in 2^-s quanta
+  const int s = min(LOW, max(0, __clz(h ^ (h >> 31)) - 2));
+  const long long m = (long long)((unsigned long long)f.hi << s) | (long long)(f.lo >> (LOW - s));  // in 2^-s quanta
   unsigned long long u = (unsigned long long)(m < 0 ? -m : m);
   const int z = __clzll((long long)u);
   u <<= z & 63;
@@ -325,19 +332,6 @@ __device__ __forceinline__ void metropolis_parts(uint32_t ua, float &lnu, float 
   const float uf = (float)ua * 2.3283064e-10f;  // a * 2^-32
   lnu = __logf(uf);
   mu = 1e-4f + 1e-8f / uf;
-}
-
-// FP64 launches hold table entries and ECI coefficients as int64 multiples of 2^-k: this part's FP64 pipe
-// issues one warp instruction in 16 cycles per SM, so the additions of an energy change in each of 16 warps
-// cost more than the rest of a round, while 64-bit integer additions are two instructions on the wide pipe,
-// and exact.  k is as large as sums of 2 n entries of magnitude `most` allow (|sum| < 2^61), i.e. the quantum
-// is at most 2^-60 n most: for 458 geometries of 0.1 eV 4e-17 eV, the spacing of FP64 numbers near 0.3 eV.
-// 0: not representable (an ECI that is infinite or NaN), everything stays FP64.
-__device__ __forceinline__ double fixed_point_scale(double most, int n) {
-  const double bound = most * 2.0 * (double)(n + 1);
-  if (!(bound < 1e300)) return 0.0;
-  if (!(bound > 1e-200)) return 1.0;
-  return ldexp(1.0, 60 - ilogb(bound));
 }
 
 // Two-state acceptance of waste recycling (Frenkel, PNAS 101, 17571 (2004);

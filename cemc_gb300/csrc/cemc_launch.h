@@ -41,6 +41,7 @@ struct RunArgs {
   int row_bits;      // scheduled kernel: log2 of the neighbour-row ring (ring_bits: trials in flight)
   int head_bits;     // scheduled kernel: log2 of the site-hash size
   int route;         // 0, or the mark in a chain's status word that leaves it to this launch (cemc_route.h)
+  int fx_low;        // table form, FP64: fixed-point entries, their low parts behind the layout (fx_low_bytes)
   int cons;          // 1: the build with the constraint redraw loop and first-move acceptance (one CTA per chain)
 };
 
@@ -189,6 +190,9 @@ __host__ __device__ inline McLayout mc_layout(const DevGeo &g, int warps, int mo
   L.total = o;
   return L;
 }
+
+// Shared memory behind a table launch's layout for the low parts of its fixed-point entries and singlet energies.
+inline size_t fx_low_bytes(const DevGeo &g) { return align16(4 * (size_t)(g.tab_len + g.n_sym * g.n_sym)); }
 
 struct SpinDev;
 cudaError_t launch_mc(const DevGeo &g, const RunArgs &a, int move, int precision, size_t smem, cudaStream_t st,

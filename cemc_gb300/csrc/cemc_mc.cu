@@ -307,6 +307,7 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
   R *ftab = reinterpret_cast<R *>(smem + L.ftab);
   uint4 *geos_s = reinterpret_cast<uint4 *>(smem + L.geos);
   constexpr bool FX = TAB && sizeof(R) == 8;  // table entries in fixed point, if they can be
+  uint32_t *ftab_low = reinterpret_cast<uint32_t *>(smem + L.total);  // their low parts (a.fx_low), then sfx's
   long long *ftab_fx = reinterpret_cast<long long *>(smem + L.ftab);
   long long *sfx_s = reinterpret_cast<long long *>(smem + L.sfx);  // [old * S + new] energy of the singlets' change
   R *vb = va + g.vals_len;
@@ -743,17 +744,24 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
   float fx_kT = 0.f;
   if constexpr (FX) {
     const int S = g.n_sym;
-    fx_scale = fixed_point_scale(table_most(g, ftab, a.eci + (size_t)chain * n_eci, lane), g.n_geo + CEMC_MAX_BF);
+    if (a.fx_low)
+      fx_scale = table_quanta(g, ftab, a.eci + (size_t)chain * n_eci, (SWAP ? 2 : 1) * g.n_geo, !SWAP, lane);
     __syncthreads();
     if (fx_scale != 0.0) {
       fx_inv = 1.0 / fx_scale;
       fx_kT = (float)(fx_inv / kT);
-      for (int i = tid; i < g.tab_len; i += blockDim.x) ftab_fx[i] = __double2ll_rn((double)ftab[i] * fx_scale);
+      for (int i = tid; i < g.tab_len; i += blockDim.x) {
+        const FxNum f = fx_of<kFxTableLow>((double)ftab[i], fx_scale);
+        ftab_fx[i] = f.hi;
+        ftab_low[i] = f.lo;
+      }
       for (int s = tid; s < S * S; s += blockDim.x) {
         double v = 0.0;
         for (int b = 0; b < g.n_bf; ++b)
           if (g.singlet_eci[b] >= 0) v += coef_s[g.singlet_eci[b]] * (bf_s[b * S + s % S] - bf_s[b * S + s / S]);
-        sfx_s[s] = __double2ll_rn(v * fx_scale);
+        const FxNum f = fx_of<kFxTableLow>(v, fx_scale);
+        sfx_s[s] = f.hi;
+        ftab_low[g.tab_len + s] = f.lo;
       }
     }
   }
@@ -800,13 +808,13 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
       if (sing != 0.0) least = fmin(least, fabs(sing));
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) least = fmin(least, __shfl_xor_sync(kFull, least, o));
-      fx_scale = fx_quanta(warp_sum(own) + 2.0 * fabs(sing), least);
+      fx_scale = fx_quanta<kFxLow>(warp_sum(own) + 2.0 * fabs(sing), least);
       if (__any_sync(kFull, (SWAP ? 2 : 1) * (sp_e.n_pairs + sp_e.n_multi) >= kFxTerms)) fx_scale = 0.0;
       if (fx_scale != 0.0) {
         fx_inv = 1.0 / fx_scale;
         fx_kT = (float)(fx_inv / kT);
-        sp_cfx = fx_of((double)sp_coef, fx_scale);
-        sing_fx = fx_of(sing, fx_scale);
+        sp_cfx = fx_of<kFxLow>((double)sp_coef, fx_scale);
+        sing_fx = fx_of<kFxLow>(sing, fx_scale);
       }
     }
     sp_multi = __ballot_sync(kFull, el < sd.n_cl && sp_e.n_multi > 0);
@@ -1041,7 +1049,7 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
           if (SFX && fx_scale != 0.0) {
             if (sd.singlet_eci >= 0 && hl == 0 && has) Dh[sd.singlet_eci] = delta;
             de_fx = fx_sum<LW>(fx_mul(sp_cfx, P), sing_fx, delta);
-            de = (R)fx_value(de_fx, fx_inv);
+            de = (R)fx_value<kFxLow>(de_fx, fx_inv);
           } else {
             R sum = sp_coef * (R)P;
 #pragma unroll
@@ -1188,27 +1196,32 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
           if constexpr (TAB) {
             __syncwarp();
             const int S = g.n_sym;
-            // energy change by the tables of type T (the swap's two sites in one pass, unless their groups differ)
-            auto change = [&](auto *F) {
+            // energy change by `sum`, table_sum or table_sum_fx (the swap's two sites in one pass, unless their
+            // groups differ: `add` of two)
+            auto change = [&](auto sum, auto add) {
               if constexpr (!SWAP)
-                return table_sum<std::remove_pointer_t<decltype(F)>, false>(S, geos_s, F, sp_a, sp_a, old_a * S + na, 0,
-                                                                           gstart_s[ga], gstart_s[ga + 1], lane);
+                return sum(std::false_type{}, sp_a, sp_a, old_a * S + na, 0, gstart_s[ga], gstart_s[ga + 1]);
               else if (ga == gb)
-                return table_sum<std::remove_pointer_t<decltype(F)>, true>(S, geos_s, F, sp_a, sp_b, A_ * S + B_,
-                                                                          B_ * S + A_, gstart_s[ga], gstart_s[ga + 1],
-                                                                          lane);
+                return sum(std::true_type{}, sp_a, sp_b, A_ * S + B_, B_ * S + A_, gstart_s[ga], gstart_s[ga + 1]);
               else
-                return table_sum<std::remove_pointer_t<decltype(F)>, false>(S, geos_s, F, sp_a, sp_a, A_ * S + B_, 0,
-                                                                           gstart_s[ga], gstart_s[ga + 1], lane) +
-                       table_sum<std::remove_pointer_t<decltype(F)>, false>(S, geos_s, F, sp_b, sp_b, B_ * S + A_, 0,
-                                                                           gstart_s[gb], gstart_s[gb + 1], lane);
+                return add(sum(std::false_type{}, sp_a, sp_a, A_ * S + B_, 0, gstart_s[ga], gstart_s[ga + 1]),
+                           sum(std::false_type{}, sp_b, sp_b, B_ * S + A_, 0, gstart_s[gb], gstart_s[gb + 1]));
             };
             if (FX && fx_scale != 0.0) {
-              de_fx.hi = change(ftab_fx);
-              if (!SWAP) de_fx.hi += sfx_s[old_a * S + na];
-              de = (R)((double)de_fx.hi * fx_inv);
+              FxNum f = change(
+                  [&](auto two, const int8_t *pa, const int8_t *pb, int on_a, int on_b, int lo, int hi) {
+                    return table_sum_fx<two.value>(S, geos_s, ftab_fx, ftab_low, pa, pb, on_a, on_b, lo, hi, lane);
+                  },
+                  [](FxNum x, FxNum y) { return FxNum{x.hi + y.hi, x.lo + y.lo}; });
+              if (!SWAP) f = FxNum{f.hi + sfx_s[old_a * S + na], f.lo + ftab_low[g.tab_len + old_a * S + na]};
+              de_fx = fx_carry<kFxTableLow>(f.hi, (int)f.lo);
+              de = (R)fx_value<kFxTableLow>(de_fx, fx_inv);
             } else {
-              de = change(ftab);
+              de = change(
+                  [&](auto two, const int8_t *pa, const int8_t *pb, int on_a, int on_b, int lo, int hi) {
+                    return table_sum<R, two.value>(S, geos_s, ftab, pa, pb, on_a, on_b, lo, hi, lane);
+                  },
+                  [](R x, R y) { return x + y; });
               if (!SWAP)
                 for (int b = 0; b < g.n_bf; ++b)
                   if (g.singlet_eci[b] >= 0)
@@ -1267,7 +1280,7 @@ __global__ void __launch_bounds__(kMcMaxThreads, 1) mc_kernel(DevGeo g, RunArgs 
             if (sd.singlet_eci >= 0 && lane == 0) Dw[sd.singlet_eci] = SWAP ? 0 : delta;
             if (SFX && fx_scale != 0.0) {
               de_fx = fx_sum<32>(fx_mul(sp_cfx, P), SWAP ? FxNum{0, 0u} : sing_fx, delta);
-              de = (R)fx_value(de_fx, fx_inv);
+              de = (R)fx_value<kFxLow>(de_fx, fx_inv);
             } else {
               R sum = warp_sum(sp_coef * (R)P);
               if (sd.singlet_eci >= 0 && !SWAP) sum += coef_s[sd.singlet_eci];

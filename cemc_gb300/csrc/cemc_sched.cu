@@ -240,12 +240,12 @@ __global__ void __launch_bounds__(kSchedMaxThreads, 1) sched_kernel(DevGeo g, Ru
       if ((double)sing != 0.0) least = fmin(least, fabs((double)sing));
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) least = fmin(least, __shfl_xor_sync(kFull, least, o));
-      const double scale = fx_quanta(most, least);
+      const double scale = fx_quanta<kFxLow>(most, least);
       if (scale != 0.0) {
         fx_inv = 1.0 / scale;
         fx_kT = (float)(fx_inv / kT);
-        coef_fx = fx_of((double)coef, scale);
-        sing_fx = fx_of((double)sing, scale);
+        coef_fx = fx_of<kFxLow>((double)coef, scale);
+        sing_fx = fx_of<kFxLow>((double)sing, scale);
       }
     }
     const bool cols = 8 * hl < cp16;  // this lane's eight columns 8 hl .. 8 hl + 7 of a row
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(kSchedMaxThreads, 1) sched_kernel(DevGeo g, Ru
         FxNum de_fx{0, 0u};
         if (FX && fx_inv != 0.0) {
           de_fx = fx_sum<8>(fx_mul(coef_fx, P), sing_fx, delta);
-          de = (R)fx_value(de_fx, fx_inv);
+          de = (R)fx_value<kFxLow>(de_fx, fx_inv);
         } else {
           R sum = coef * (R)P;
 #pragma unroll

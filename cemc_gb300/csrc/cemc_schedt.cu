@@ -95,6 +95,7 @@ __global__ void __launch_bounds__(32 * (WARPS + kTickHelpers), 1) tick_kernel(De
   int32_t *gstart_s = reinterpret_cast<int32_t *>(smem + L.gstart);
   R *ftab = reinterpret_cast<R *>(smem + L.ftab);
   long long *ftab_fx = reinterpret_cast<long long *>(smem + L.ftab);
+  uint32_t *ftab_low = reinterpret_cast<uint32_t *>(smem + L.total);  // low parts (a.fx_low), then sfx's
   uint4 *geos_s = reinterpret_cast<uint4 *>(smem + L.geos);
   long long *sfx_s = reinterpret_cast<long long *>(smem + L.sfx);  // [old * S + new] energy of the singlets' change
   A *lacc0 = reinterpret_cast<A *>(smem + L.acc);
@@ -191,17 +192,24 @@ __global__ void __launch_bounds__(32 * (WARPS + kTickHelpers), 1) tick_kernel(De
   double fx_scale = 0.0, fx_inv = 0.0;  // FP64: table entries are multiples of fx_inv (0: they are FP64)
   float fx_kT = 0.f;
   if constexpr (FX) {
-    fx_scale = fixed_point_scale(table_most(g, ftab, a.eci + (size_t)chain * n_eci, lane), g.n_geo + CEMC_MAX_BF);
+    if (a.fx_low)
+      fx_scale = table_quanta(g, ftab, a.eci + (size_t)chain * n_eci, (SWAP ? 2 : 1) * g.n_geo, !SWAP, lane);
     __syncthreads();
     if (fx_scale != 0.0) {
       fx_inv = 1.0 / fx_scale;
       fx_kT = (float)(fx_inv / kT);
-      for (int i = tid; i < g.tab_len; i += blockDim.x) ftab_fx[i] = __double2ll_rn((double)ftab[i] * fx_scale);
+      for (int i = tid; i < g.tab_len; i += blockDim.x) {
+        const FxNum f = fx_of<kFxTableLow>((double)ftab[i], fx_scale);
+        ftab_fx[i] = f.hi;
+        ftab_low[i] = f.lo;
+      }
       for (int s = tid; s < S * S; s += blockDim.x) {
         double v = 0.0;
         for (int b = 0; b < n_bf; ++b)
           if (g.singlet_eci[b] >= 0) v += coef_s[g.singlet_eci[b]] * (bf_s[b * S + s % S] - bf_s[b * S + s / S]);
-        sfx_s[s] = __double2ll_rn(v * fx_scale);
+        const FxNum f = fx_of<kFxTableLow>(v, fx_scale);
+        sfx_s[s] = f.hi;
+        ftab_low[g.tab_len + s] = f.lo;
       }
     }
     __syncthreads();
@@ -288,32 +296,41 @@ __global__ void __launch_bounds__(32 * (WARPS + kTickHelpers), 1) tick_kernel(De
             ga = SWAP ? (int)g.site_group[sa] : (int)d.grp;
             if (SWAP) gb = g.site_group[sb];
           }
-          // energy change by the tables of type T (the swap's two sites in one pass, unless their groups differ)
-          auto change = [&](auto *F) {
-            using T = std::remove_pointer_t<decltype(F)>;
+          // energy change by `sum`, table_sum or table_sum_fx (the swap's two sites in one pass, unless their groups
+          // differ: `add` of two)
+          auto change = [&](auto sum, auto add) {
             const int on_a = oa * S + na, on_b = na * S + oa;
             if constexpr (!SWAP)
-              return table_sum<T, false>(S, geos_s, F, sp_a, sp_a, on_a, 0, gstart_s[ga], gstart_s[ga + 1], lane);
+              return sum(std::false_type{}, sp_a, sp_a, on_a, 0, gstart_s[ga], gstart_s[ga + 1]);
             else if (ga == gb)
-              return table_sum<T, true>(S, geos_s, F, sp_a, sp_b, on_a, on_b, gstart_s[ga], gstart_s[ga + 1], lane);
-            return table_sum<T, false>(S, geos_s, F, sp_a, sp_a, on_a, 0, gstart_s[ga], gstart_s[ga + 1], lane) +
-                   table_sum<T, false>(S, geos_s, F, sp_b, sp_b, on_b, 0, gstart_s[gb], gstart_s[gb + 1], lane);
+              return sum(std::true_type{}, sp_a, sp_b, on_a, on_b, gstart_s[ga], gstart_s[ga + 1]);
+            return add(sum(std::false_type{}, sp_a, sp_a, on_a, 0, gstart_s[ga], gstart_s[ga + 1]),
+                       sum(std::false_type{}, sp_b, sp_b, on_b, 0, gstart_s[gb], gstart_s[gb + 1]));
           };
           R de;
-          long long de_fx = 0;  // the energy change in units of fx_inv
+          FxNum de_fx{0, 0u};  // the energy change in units of fx_inv
           if (FX && fx_scale != 0.0) {
-            de_fx = change(ftab_fx);
-            if (!SWAP) de_fx += sfx_s[oa * S + na];
-            de = (R)((double)de_fx * fx_inv);
+            FxNum f = change(
+                [&](auto two, const int8_t *pa, const int8_t *pb, int on_a, int on_b, int lo, int hi) {
+                  return table_sum_fx<two.value>(S, geos_s, ftab_fx, ftab_low, pa, pb, on_a, on_b, lo, hi, lane);
+                },
+                [](FxNum x, FxNum y) { return FxNum{x.hi + y.hi, x.lo + y.lo}; });
+            if (!SWAP) f = FxNum{f.hi + sfx_s[oa * S + na], f.lo + ftab_low[g.tab_len + oa * S + na]};
+            de_fx = fx_carry<kFxTableLow>(f.hi, (int)f.lo);
+            de = (R)fx_value<kFxTableLow>(de_fx, fx_inv);
           } else {
-            de = change(ftab);
+            de = change(
+                [&](auto two, const int8_t *pa, const int8_t *pb, int on_a, int on_b, int lo, int hi) {
+                  return table_sum<R, two.value>(S, geos_s, ftab, pa, pb, on_a, on_b, lo, hi, lane);
+                },
+                [](R x, R y) { return x + y; });
             if (!SWAP)
               for (int b = 0; b < n_bf; ++b)
                 if (g.singlet_eci[b] >= 0)
                   de += coef_s[g.singlet_eci[b]] * (bf_s[b * S + na] - bf_s[b * S + oa]);
           }
           if (lane == 0) {
-            const int acc = FX && fx_scale != 0.0 ? metropolis_fx(FxNum{de_fx, 0u}, (double)de, d.ua, d.ub, kT, fx_kT)
+            const int acc = FX && fx_scale != 0.0 ? metropolis_fx(de_fx, (double)de, d.ua, d.ub, kT, fx_kT)
                                                   : metropolis<R>(de, d.ua, d.ub, kT, inv_kT);
             if (acc) {
               occ[sa] = (int8_t)na;

@@ -31,21 +31,31 @@ __device__ inline double table_entry(const DevGeo &g, const double *eci, int idx
   return v;
 }
 
-// Largest magnitude of a chain's table entries and singlet energies (one warp; NaN counts as infinite).
+// Fixed-point quanta of a chain's tables (fx_quanta; one warp): `n` entries at most make up an energy change, and with
+// `singlets` (flips) the singlets' change.  NaN counts as infinite.
 template <typename R>
-__device__ inline double table_most(const DevGeo &g, const R *ftab, const double *eci, int lane) {
+__device__ inline double table_quanta(const DevGeo &g, const R *ftab, const double *eci, int n, bool singlets, int lane) {
   const int S = g.n_sym;
-  double most = 0.0;
+  double most = 0.0, alone = 0.0, least = HUGE_VAL;
   for (int i = lane; i < g.tab_len; i += 32) most = fmax(most, isnan((double)ftab[i]) ? HUGE_VAL : fabs((double)ftab[i]));
-  for (int i = lane; i < g.n_eci; i += 32)
-    if (g.eci_kind[i] == 1) {
-      const double *bf = g.bf + g.eci_dec[i] * S;
-      for (int s = 0; s < S * S; ++s)
-        most = fmax(most, isnan(eci[i]) ? HUGE_VAL : fabs(eci[i] * (bf[s % S] - bf[s / S])));
+  for (int k = lane; k < g.n_eci; k += 32) {
+    const int kind = g.eci_kind[k];
+    if (kind == 0 || (kind == 1 && !singlets)) continue;
+    const double c = kind == 2 ? fabs(eci[k] * (double)g.n_sites * g.eci_w[k]) : fabs(eci[k]);
+    if (c > 0.0) least = fmin(least, c);
+    if (kind == 1) {
+      const double *bf = g.bf + g.eci_dec[k] * S;
+      double d = 0.0;
+      for (int s = 0; s < S * S; ++s) d = fmax(d, fabs(bf[s % S] - bf[s / S]));
+      alone += isnan(c) ? HUGE_VAL : c * d;
     }
+  }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) most = fmax(most, __shfl_xor_sync(kFull, most, o));
-  return most;
+  for (int o = 16; o > 0; o >>= 1) {
+    most = fmax(most, __shfl_xor_sync(kFull, most, o));
+    least = fmin(least, __shfl_xor_sync(kFull, least, o));
+  }
+  return fx_quanta<kFxTableLow>((double)n * most + warp_sum(alone), least);
 }
 
 // Energy change of one flip (or, TWO, of a swap's two flips) from the pattern
@@ -54,7 +64,7 @@ __device__ inline double table_most(const DevGeo &g, const R *ftab, const double
 // Geometries [lo, hi) are those of the changed site's translation group, packed as
 // {c1 | c2 << 8 | c3 << 16, off, S^m, 0}.  Lane l adds geometries lo + l, lo + l + 32, .. in this order, then a butterfly.
 //
-// T is the entries' type: float, double, or int64 fixed-point (FP64 launches; see fixed_point_scale()).
+// T is the entries' type, float or double; table_sum_fx() is the same for entries in fixed point (FP64 launches).
 // (Four lookups in flight at a time, with the geometries in shared memory or in registers, measured slower:
 // ladder 34.1 -> 35.1 and 43 ms, the loop is bound by its shared-memory wavefronts and instructions.)
 template <typename T, bool TWO>
@@ -70,6 +80,32 @@ __device__ __forceinline__ T table_sum(int S, const uint4 *geos, const T *F, con
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
+  return sum;
+}
+
+// table_sum() of entries in fixed point, their low parts in an array of their own; the sum's low part is not carried.
+template <bool TWO>
+__device__ __forceinline__ FxNum table_sum_fx(int S, const uint4 *geos, const long long *F, const uint32_t *low,
+                                              const int8_t *spa, const int8_t *spb, int on_a, int on_b, int lo, int hi,
+                                              int lane) {
+  const int S2 = S * S;
+  FxNum sum{0, 0u};
+  for (int i = lo + lane; i < hi; i += 32) {
+    const uint4 e = geos[i];
+    const int c1 = e.x & 0xff, c2 = (e.x >> 8) & 0xff, c3 = (e.x >> 16) & 0xff;
+    const uint32_t at = e.y + on_a * e.z + spa[c1] + S * spa[c2] + S2 * spa[c3];
+    sum.hi += F[at];
+    sum.lo += low[at];
+    if (TWO) {
+      const uint32_t bt = e.y + on_b * e.z + spb[c1] + S * spb[c2] + S2 * spb[c3];
+      sum.hi += F[bt];
+      sum.lo += low[bt];
+    }
+  }
+  sum.hi += (long long)(sum.lo >> kFxTableLow);
+  sum.lo = __reduce_add_sync(kFull, sum.lo & ((1u << kFxTableLow) - 1u));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum.hi += __shfl_xor_sync(kFull, sum.hi, o);
   return sum;
 }
 
