@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(32 * (WARPS + kTickHelpers), 1) tick_kernel(De
     }
   }
   __syncthreads();
-  if (*fault_s) {  // the chain's trial counter and sums are not written
+  if (*fault_s) {  // only the site lists hold moves of this launch (a host that goes on rebuilds them)
     if (tid == 0 && a.status) a.status[chain] = CEMC_ERR_INTERNAL;
     return;
   }

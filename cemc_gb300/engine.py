@@ -370,8 +370,19 @@ class ChainBatch:
     def check_status(self):
         st = self.status.cpu().numpy()
         if np.any(st != 0):
+            if self.trk is not None and np.any(st == _lib.ERR_INTERNAL):
+                self._restore_lists(np.nonzero(st == _lib.ERR_INTERNAL)[0])
             bad = int(np.nonzero(st)[0][0])
             raise _lib.CemcError(int(st[bad]), "chain %d reported a device status" % bad)
+
+    def _restore_lists(self, chains):
+        """Site lists of chains whose launch was stopped by a consistency check, from their occupations: the lists may
+        hold moves that the occupation does not."""
+        m = self.geo.model
+        idx = torch.as_tensor(chains, device=self.occ.device)
+        lists = build_tracker(self.occ[idx].cpu().numpy(), m.n_sym, m.background)
+        for t, v in zip((self.trk, self.loc, self.trk_start, self.trk_count), lists):
+            t[idx] = torch.as_tensor(v).to(t.device)
 
     # -- accumulators --------------------------------------------------------
     def reset_accumulators(self, e_ref=None):

@@ -28,7 +28,10 @@ extern "C" {
 #define CEMC_ERR_STATE 4      /* move inconsistent with the current occupation (ce_updater.cpp:530-537) */
 #define CEMC_ERR_LIMIT 5      /* a compiled-in limit was exceeded */
 #define CEMC_ERR_TIMEOUT 6    /* a bounded device wait ran out */
-#define CEMC_ERR_INTERNAL 7   /* a device-side consistency check failed (the chain's state was not written) */
+#define CEMC_ERR_INTERNAL 7   /* a device-side consistency check failed.  Correlation functions, energy, trial counter and
+                                 running sums were not written.  The site lists of a swap chain, and the occupation
+                                 of one that does not fit in shared memory, are changed move by move in device memory
+                                 and may hold moves of the stopped launch: rebuild the lists from the occupation */
 #define CEMC_ERR_NO_MOVE 8    /* no trial move satisfying the move constraints within max_attempts draws
                                  (CanNotFindLegalMoveError, montecarlo.py:984-987) */
 
