@@ -1,7 +1,7 @@
 #!/usr/bin/env bash
 # Build the reference's own CEUpdater (CEMC, cpp/src) as a test oracle.
 #
-# Reads the reference sources where they lie (default /root/reference, or $1)
+# Reads the reference sources where they lie ($1, or the folder that CEMC_REFERENCE names)
 # and writes ONLY into oracle/_ref/.  It does not run the reference's setup.py:
 # it compiles the eleven CEUpdater sources with the reference's own flags
 # (-std=c++11 -fopenmp -O3, setup.py:34) and wraps them with the reference's
@@ -11,11 +11,11 @@
 # Needs cython, g++, Python and numpy headers; exits 0 with a message when the
 # reference tree is absent (as on machines that only run the product).
 set -euo pipefail
-REF=${1:-${CEMC_REFERENCE:-/root/reference}}
+REF=${1:-${CEMC_REFERENCE:-}}
 HERE=$(cd "$(dirname "$0")" && pwd)
 OUT="$HERE/_ref"
-if [ ! -d "$REF/cpp/src" ]; then
-  echo "build_ref: reference sources not found at $REF; skipping"
+if [ -z "$REF" ] || [ ! -d "$REF/cpp/src" ]; then
+  echo "build_ref: reference sources not found at '${REF}'; skipping"
   exit 0
 fi
 command -v cython >/dev/null || { echo "build_ref: cython not available; skipping"; exit 0; }
