@@ -113,12 +113,14 @@ def load():
         L.cemc_apply_changes.argtypes = [_P, _P, _P, _P, _P, C.c_int32, _P, _P, _P, _P, _P]
         L.cemc_calculate.argtypes = [_P, _P, _P, _P, _P, C.c_int32, _P, _P, _P, _P, _P]
         L.cemc_revert.argtypes = [_P, _P, _P, _P, _P, _P, C.c_int32, _P, _P, _P]
+        L.cemc_decide.argtypes = L.cemc_run_decided.argtypes = L.cemc_run.argtypes
         L.cemc_read.argtypes = [_P, _P, C.c_size_t, _P]
         L.cemc_delta_e.argtypes = [_P, _P, _P, C.c_int32, C.c_int32, C.c_int32, C.c_int32, _P, _P, _P]
         L.cemc_pt_exchange.argtypes = [C.c_int32, C.c_int32, C.c_uint64, C.c_uint64, _P, _P, _P, _P, _P, _P]
         L.cemc_last_error.argtypes = [C.c_char_p, C.c_size_t]
         L.cemc_version.argtypes = [C.POINTER(C.c_int32)] * 3
-        for name in ("cemc_geometry_create", "cemc_geometry_destroy", "cemc_run", "cemc_recompute", "cemc_energy",
+        for name in ("cemc_geometry_create", "cemc_geometry_destroy", "cemc_run", "cemc_decide", "cemc_run_decided",
+                     "cemc_recompute", "cemc_energy",
                      "cemc_recompute_noalloc",
                      "cemc_apply_changes", "cemc_calculate", "cemc_revert", "cemc_read", "cemc_delta_e",
                      "cemc_pt_exchange", "cemc_last_error", "cemc_version"):
@@ -138,7 +140,7 @@ def exported_symbols():
     """Names declared in include/cemc_gb300.h that the loaded library exports."""
     L = load()
     names = []
-    for n in ("cemc_geometry_create", "cemc_geometry_destroy", "cemc_geometry_device_bytes", "cemc_run",
+    for n in ("cemc_geometry_create", "cemc_geometry_destroy", "cemc_geometry_device_bytes", "cemc_run", "cemc_decide", "cemc_run_decided",
               "cemc_recompute_scratch_doubles", "cemc_stamp_words", "cemc_recompute", "cemc_recompute_noalloc", "cemc_energy", "cemc_apply_changes",
               "cemc_calculate", "cemc_revert", "cemc_read", "cemc_delta_e", "cemc_pt_exchange", "cemc_last_error",
               "cemc_version"):

@@ -52,9 +52,11 @@ class BatchRunner:
     def n_chains(self) -> int:
         return self.cb.n_chains
 
-    def _step_body(self, with_recompute: bool):
+    def _step_body(self, with_recompute: bool, part: str = "cemc_run"):
         self.cb.run(self.trials_per_step, precision=self.precision, warps=self.warps, cluster=self.cluster,
-                    kernel=self.kernel)
+                    kernel=self.kernel, part=part)
+        if part == "cemc_decide":
+            return
         if with_recompute and not self.cb.recomputed:
             self.cb.recompute()
 
@@ -151,7 +153,8 @@ class MultiBatchRunner:
     stream.  The captured step forks every group's stream from a capture stream,
     records each group's MC launch and recompute on it, and joins them back, so
     ONE graph launch runs all groups' kernels concurrently on the device (uneven
-    supercells do not wait for one another).  ``trials`` counts the step's
+    supercells do not wait for one another), after a second, small graph where kernels
+    are chosen on the device.  ``trials`` counts the step's
     trials over all groups.
     """
 
@@ -175,14 +178,14 @@ class MultiBatchRunner:
         before the short ones take the SMs, and the short ones fill the SMs around them."""
         return sorted(self.runners, key=lambda r: -r.trials_per_step * (2 if r.geo.model.n_sym > 2 else 1))
 
-    def _body(self):
+    def _body(self, part: str):
         start = torch.cuda.Event()
         start.record(self.stream)
         done = []
         for r in self._launch_order():
             r.stream.wait_event(start)
             with torch.cuda.stream(r.stream):
-                r._step_body(r.recompute_every == 1)
+                r._step_body(r.recompute_every == 1, part)
             ev = torch.cuda.Event()
             ev.record(r.stream)
             done.append(ev)
@@ -194,13 +197,20 @@ class MultiBatchRunner:
             return
         snaps = [r.snapshot() for r in self.runners]
         with torch.cuda.stream(self.stream):
-            self._body()  # warm the launch path outside the capture
+            self._body("cemc_run")  # warm the launch path outside the capture
         for r, snap in zip(self.runners, snaps):
             r.restore(snap)
         torch.cuda.synchronize()
+        # kernels chosen on the device are chosen by a graph of its own ahead of the step's, whose first kernels
+        # then start in the order of their launches
+        self._decisions = None
+        if any(r.cb.last_scheduled == 2 for r in self.runners):
+            self._decisions = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(self._decisions, stream=self.stream):
+                self._body("cemc_decide")
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g, stream=self.stream):
-            self._body()
+            self._body("cemc_run_decided")
         self._graph = g
 
     def step(self, n: int = 1):
@@ -209,6 +219,8 @@ class MultiBatchRunner:
             self.capture()
         for _ in range(n):
             with torch.cuda.stream(self.stream):
+                if self._decisions is not None:
+                    self._decisions.replay()
                 self._graph.replay()
             for r in self.runners:
                 r.steps_done += 1

@@ -1110,7 +1110,10 @@ void fit_tick(const cemc_geometry *geo, int precision, int move, int part, int b
 
 }  // namespace
 
-extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream) {
+// The choice between kernels that a call leaves to the device: taken in the call, alone, or taken before it.
+enum class Decision { kHere, kOnly, kBefore };
+
+static int run(const cemc_geometry *geo, cemc_run_desc *r, void *stream, Decision decision) {
   if (!geo || !r) return fail(CEMC_ERR_ARG, "null geometry or run descriptor");
   const cemc::DevGeo &g = geo->g;
   if (r->n_chains <= 0) return fail(CEMC_ERR_ARG, "no chains");
@@ -1182,6 +1185,7 @@ extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream
       smem = cemc::field_layout(g, fd.n_cl, fd.pw, fd.n_cnt, fd.n_upd, rs, fa.ring_bits, true).total;
     }
     if (smem <= (size_t)geo->max_smem) {
+      if (decision == Decision::kOnly) return CEMC_OK;
       fa.seed = r->seed;
       fa.occ = r->occ;
       fa.cf = r->cf;
@@ -1367,12 +1371,13 @@ extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream
   Scheduled sch;
   sch.args = a;
   const bool exact = a.gstamp || a.stamp_bits == exact_bits;
+  const int beside = std::max(0, r->beside);
   const bool flips = form == cemc::kFormSpin && r->move == CEMC_MOVE_FLIP;  // else the table form's moves
   if (flips && geo->spin.qtr_ok && g.table16 && !constrained && exact && r->cluster != 2 &&
       (r->kernel == CEMC_KERNEL_AUTO || r->kernel == CEMC_KERNEL_SPIN_QUARTER))
-    fit_sched(geo, r->precision, cemc::round_trials(1, a.warps, a.tpw), L.total, std::max(0, r->beside), sch);
+    fit_sched(geo, r->precision, cemc::round_trials(1, a.warps, a.tpw), L.total, beside, sch);
   else if (form == cemc::kFormTable && !constrained && exact)
-    fit_tick(geo, r->precision, r->move, cemc::round_trials(a.cl, a.warps, a.tpw), std::max(0, r->beside), sch);
+    fit_tick(geo, r->precision, r->move, cemc::round_trials(a.cl, a.warps, a.tpw), beside, sch);
   if (sch.how == Scheduled::kRouted && (!r->status || r->n_trials < cemc::kRouteTrials)) sch.how = Scheduled::kNo;
   // The table form leaves correlation functions to a full recompute at the end of the call.
   double *rscratch = nullptr;
@@ -1407,10 +1412,11 @@ extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream
     a.n_trials = sch.args.n_trials = n;
     a.chunk_offset = sch.args.chunk_offset = done;
     cudaError_t e;
-    if (sch.how == Scheduled::kRouted) {
+    if (sch.how == Scheduled::kRouted && (decision != Decision::kBefore || done > 0)) {
       e = cemc::launch_route(g, a, is_swap, sch.route, st);
       if (e != cudaSuccess) return cuda_fail(e, "route kernel launch");
     }
+    if (decision == Decision::kOnly) return CEMC_OK;
     if (sch.how) {
       e = flips ? cemc::launch_sched(g, sch.args, r->precision, sch.smem, st, geo->spin)
                 : cemc::launch_tick(g, sch.args, r->move, r->precision, sch.smem, st);
@@ -1431,6 +1437,18 @@ extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream
                   : (form == cemc::kFormGeneric || form == cemc::kFormRecycle) ? CEMC_KERNEL_GENERIC
                   : (a.tpw == 4 || sch.how == Scheduled::kAlways ? CEMC_KERNEL_SPIN_QUARTER : a.tpw == 2 ? CEMC_KERNEL_SPIN_HALFWARP : CEMC_KERNEL_SPIN);
   return CEMC_OK;
+}
+
+extern "C" int cemc_run(const cemc_geometry *geo, cemc_run_desc *r, void *stream) {
+  return run(geo, r, stream, Decision::kHere);
+}
+
+extern "C" int cemc_decide(const cemc_geometry *geo, cemc_run_desc *r, void *stream) {
+  return run(geo, r, stream, Decision::kOnly);
+}
+
+extern "C" int cemc_run_decided(const cemc_geometry *geo, cemc_run_desc *r, void *stream) {
+  return run(geo, r, stream, Decision::kBefore);
 }
 
 extern "C" size_t cemc_recompute_scratch_doubles(const cemc_geometry *geo, int32_t n_chains) {

@@ -304,7 +304,7 @@ class ChainBatch:
     def run(self, n_trials: int, precision: int = PREC_F64, warps: int = 0, trace: bool = False,
             chain_trials: Optional[torch.Tensor] = None, kernel: int = 0, cluster: int = 0,
             site_allow: Optional[torch.Tensor] = None, frozen: Optional[torch.Tensor] = None,
-            max_attempts: int = 0, accept_first: bool = False, recycle_waste: bool = False):
+            max_attempts: int = 0, accept_first: bool = False, recycle_waste: bool = False, part: str = "cemc_run"):
         """Run ``n_trials`` trials on every chain in one launch (``cemc_run``).
 
         ``chain_trials`` (device int64, one per chain, each <= n_trials) gives chains their own counts.
@@ -314,6 +314,7 @@ class ChainBatch:
         not change), ``max_attempts`` redraws per trial (0 = 10000); see ``mc_constraints``.
         ``accept_first``: the first trial of the call is accepted outright (every chain).
         ``recycle_waste``: waste-recycled acceptance and running sums (generic form, one CTA).
+        ``part``: the entry point, ``cemc_run`` or its two parts (``cemc_decide``, then ``cemc_run_decided``).
         """
         if site_allow is not None:
             if site_allow.dtype != torch.uint8 or site_allow.numel() != self.n_chains * self.geo.model.n_sites:
@@ -337,7 +338,9 @@ class ChainBatch:
                          0, 0, _ptr(site_allow), _ptr(frozen), int(max_attempts), int(bool(accept_first)),
                          int(bool(recycle_waste)), int(self.beside))
         with torch.cuda.device(self.occ.device):
-            _lib.check(self.geo.L.cemc_run(self.geo.handle, C.byref(d), _stream_ptr(self.stream)))
+            _lib.check(getattr(self.geo.L, part)(self.geo.handle, C.byref(d), _stream_ptr(self.stream)))
+        if part == "cemc_decide":
+            return None
         # the table form ends the call with a full recompute (cf and energy exact already)
         self.last_kernel = int(d.kernel_used)
         self.last_scheduled = int(d.scheduled)  # 1: a scheduled kernel ran it, 2: the device chose

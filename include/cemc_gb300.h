@@ -237,6 +237,14 @@ typedef struct {
  * clear_history, ce_updater.cpp:313-555). */
 int cemc_run(const cemc_geometry *geo, cemc_run_desc *run, void *stream);
 
+/* cemc_run in two parts, for launches whose order of start matters (several batches, the longest chains first): where
+ * cemc_run leaves the choice of the kernel to the device (scheduled = 2), cemc_decide() enqueues the decision alone,
+ * which marks the chains' status words, and cemc_run_decided() with the same descriptor, after it on the stream and
+ * with nothing of these chains in between, the kernels.  Elsewhere cemc_decide() does nothing and cemc_run_decided()
+ * is cemc_run().  No reference counterpart. */
+int cemc_decide(const cemc_geometry *geo, cemc_run_desc *run, void *stream);
+int cemc_run_decided(const cemc_geometry *geo, cemc_run_desc *run, void *stream);
+
 /* Words of a cemc_run_desc.stamps buffer for n_chains chains of this geometry:
  * two exact tables of 2^ceil(log2 N) entries per chain.  No reference counterpart
  * (the reference evaluates one trial at a time and needs no conflict test). */

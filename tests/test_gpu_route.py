@@ -155,3 +155,38 @@ def test_other_cells_and_flips(kind, move, prec, cluster):
         got.append(_left(E, cb, 5000, accepted))
     for x, y in zip(*got):
         assert torch.equal(x, y)
+
+
+def test_decision_ahead_of_the_launch():
+    """cemc_decide and cemc_run_decided are cemc_run; several batches stepped together decide ahead of their launches."""
+    from cemc_gb300 import engine as E
+    from cemc_gb300.batch import BatchRunner, MultiBatchRunner
+    a, b, c = _batch(E, 9, (4, 2, 1), 2, E.MOVE_FLIP, 3)
+    for cb, accepted in ((a, 4000), (b, 4000), (c, 0)):
+        _counters(E, cb, 5000, accepted)
+    kw = dict(precision=E.PREC_F32, warps=16, cluster=1)
+    a.run(3000, **kw)
+    for cb in (b, c):
+        cb.run(3000, part="cemc_decide", **kw)
+        torch.cuda.synchronize()
+        assert cb.trial.tolist() == [0, 0, 0]  # nothing has run
+        cb.run(3000, part="cemc_run_decided", **kw)
+    left = [_left(E, cb, 5000, accepted) for cb, accepted in ((a, 4000), (b, 4000), (c, 0))]
+    for other in left[1:]:
+        for x, y in zip(left[0], other):
+            assert torch.equal(x, y)
+    runners = [BatchRunner(cb.geo, cb.occ.cpu().numpy(), cb.eci.cpu().numpy(), 700.0, move, seed=5, warps=8, cluster=1,
+                           chain_keys=np.arange(3))
+               for cb, move in ((a, E.MOVE_FLIP), (_batch(E, 14, (2, 1, 0), 3, E.MOVE_SWAP, 3)[0], E.MOVE_SWAP),
+                                (_batch(E, 5, (2, 1, 0), 2, E.MOVE_FLIP, 3)[0], E.MOVE_FLIP))]
+    alone = [BatchRunner(r.geo, r.cb.occ.cpu().numpy(), r.cb.eci.cpu().numpy(), 700.0, r.cb.move, seed=5, warps=8, cluster=1,
+                         chain_keys=np.arange(3)) for r in runners]
+    multi = MultiBatchRunner(runners)
+    multi.step(3)
+    multi.synchronize()
+    for r, s in zip(runners, alone):
+        s.step(3)
+        s.synchronize()
+        r.cb.check_status()
+        for k in ("occ", "cf", "energy", "trial", "accum"):
+            assert torch.equal(getattr(r.cb, k).view(torch.uint8), getattr(s.cb, k).view(torch.uint8)), k
