@@ -122,13 +122,13 @@ def tune_on(cb, precision: int, shapes=None, sweeps: float = 0.25) -> Dict[tuple
 
 
 def _pick(rates: Dict[tuple, float]) -> tuple:
-    """The first shape, in the order they were timed, within 2 % of the fastest.
+    """The first shape, in the order they were timed, within 1 % of the fastest.
 
     Several shapes can be one launch (a scheduled kernel takes the round width for its running sums only), so the
     noise of the timing would choose between them, and with the width the rounding of FP32 running sums.
     """
     most = max(rates.values())
-    return next(shape for shape, rate in rates.items() if rate >= 0.98 * most)
+    return next(shape for shape, rate in rates.items() if rate >= 0.99 * most)
 
 
 def best_config(geo, move: int, precision: int, n_chains: int, batch=None) -> Tuple[int, int, int]:
