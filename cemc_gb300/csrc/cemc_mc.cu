@@ -59,7 +59,7 @@
 // their own build.  200 chains of 864 sites, 20 sweeps, FP32: 4.89 -> 3.97 ms; 100 chains of 2,048
 // sites by 16 warps, 5 sweeps: 2.40 -> 2.00 ms.  Swaps: the fetcher turns a draw into species, list slots
 // and the acceptance test's parts, and one reduction gives the two sites' differences of counts: one
-// FP64 chain of 2,048 sites, 10 sweeps, 13.0 -> 10.1 ms.
+// FP64 chain of 2,048 sites, 10 sweeps, 13.0 -> 10.1 ms (10.4 with coefficients in fixed point to their last bit).
 #include <cuda_runtime.h>
 
 #include <type_traits>

@@ -31,7 +31,8 @@
 // Bound: instruction issue.  150 warp instructions a trial, a third each for the evaluation, the lookups
 // and the helpers, at 2.0 of 4 a cycle; shared-memory wavefronts are at 40 % of their rate.  A tick takes
 // about 4,500 cycles for 58 trials (82 cycles a trial; mc_kernel's rounds: 3,500 for 22 to 30 commits).
-// Headline batch (64 chains x 16384 sites, 10 sweeps): 12.4 ms in mc_kernel's quarter-warp form, 6.4 ms here.
+// Headline batch (64 chains x 16384 sites, 10 sweeps): 12.4 ms in mc_kernel's quarter-warp form, 6.4 ms here.  Small cells
+// of chains that accept little, and more of them than SMs, are faster there: see the rule in cemc_abi.cu, cemc_route.h.
 #include <cuda_runtime.h>
 
 #include <type_traits>

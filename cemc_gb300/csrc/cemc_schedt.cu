@@ -29,8 +29,9 @@
 // of their rate.  A tick takes 7,000 to 9,000 cycles for 15 to 23 trials.  Half-warps with two trials per
 // warp (twice the instructions per warp) took twice as long per tick; geometries of 8 bytes, both rows'
 // species side by side, or separate loops for one, two and three members were slower than the plain loop.
-// 48 x 131072-site binary ladder, one sweep: 34.1 -> 29.6 ms, on half the SMs; 64 uneven ternary chains: 7.2
-// -> 4.7 ms a step (the longest chain alone 19.5 -> 13.6); 32 ternary flip chains of 4000 sites 4.42 -> 3.77 ms.
+// 48 x 131072-site binary ladder, one sweep: 34.1 -> 29.8 ms, on half the SMs; 64 uneven ternary chains, one sweep: 19.5
+// -> 13.7 ms a step, which is the longest chain's (55,296 sites), 7.2 -> 4.8 ms where the steps of three such batches
+// overlap; 32 ternary flip chains of 4000 sites 4.42 -> 3.78 ms.  Where it is not the faster one: cemc_route.h.
 #include <cuda_runtime.h>
 
 #include <type_traits>

@@ -167,7 +167,10 @@ typedef struct {
                                    NULL = n_trials for every chain; lets a batch mix jobs with different budgets */
   int32_t kernel;      /* CEMC_KERNEL_*: which implementation runs the trials */
   int32_t cluster;     /* CTAs per chain: 1, 2 (a thread-block cluster pair on two SMs, twice the trials
-                          per round), or 0 = 2 when every chain's pair fits on the GPU at once, else 1 */
+                          per round), or 0 = 2 when every chain's pair fits on the GPU at once, else 1.  The
+                          scheduled table kernel runs one CTA per chain whatever is asked for; 2 then means the
+                          width of the rounds the running sums are taken in, and is refused where a pair does not
+                          fit.  An explicit 2 keeps spin flips out of the scheduled flip kernel */
   double *scratch;     /* table kernel: buffer for the final recompute, at least cemc_recompute_scratch_doubles()
                           doubles (a smaller buffer is refused with CEMC_ERR_ARG).  NULL = the fixed array
                           behind cemc_recompute_noalloc(), under the same rules: at most 1048576 doubles
@@ -209,16 +212,22 @@ typedef struct {
  * for — else the table form when its tables fit, else the generic form.  All
  * give the same decisions for the same stream.  The spin forms evaluate a
  * trial from a bit-packed neighbourhood (popcounts of shell masks, parities of
- * multi-site terms), one trial per warp, per 16 or per 8 lanes; unconstrained
- * flips of cells with enough sites, asked for as AUTO or SPIN_QUARTER, run in
- * the scheduled kernel (trials that do not touch one another in any order; one
- * per 8 lanes; kernel_used reports SPIN_QUARTER, and `warps` keeps its meaning
- * only for the rounds the running sums are taken in); the generic form
+ * multi-site terms), one trial per warp, per 16 or per 8 lanes; the generic form
  * multiplies basis values term by term and keeps the correlation functions up
  * to date trial by trial; the table form looks up one precomputed energy change
  * per cluster geometry (tables built per chain from its ECIs at launch) and
  * brings correlation functions and energies up to date with a full recompute
- * at the end of the call (run desc `scratch`). */
+ * at the end of the call (run desc `scratch`).
+ *
+ * Unconstrained spin flips asked for as AUTO or SPIN_QUARTER, and unconstrained
+ * moves of the table form, have a scheduled kernel each (trials that do not
+ * touch one another, in any order).  It runs cells of enough sites: always
+ * where it is the faster one for any state, by the acceptance in `accum` and the
+ * composition where that depends on the state (calls of at least 2048 trials
+ * a chain with `status` given), never below 32 neighbourhoods.  It leaves the
+ * same bits; `scheduled` reports it, kernel_used names the form (SPIN_QUARTER
+ * for flips that are always scheduled), and `warps` then has its meaning only for
+ * the rounds the running sums are taken in. */
 #define CEMC_KERNEL_AUTO 0
 #define CEMC_KERNEL_GENERIC 1
 #define CEMC_KERNEL_SPIN 2
